@@ -1631,27 +1631,46 @@ static void decompress(const uint8_t* d_in, size_t bytes, uint32_t nx, uint32_t 
     decode_finish<T>(uint32_t(pin[8]), d_in, h, L, g, P.status, P.seen, stream);
 }
 
+// Pinned host staging that grows on demand.
+struct PinnedBuffer {
+    void* ptr = nullptr;
+    size_t cap = 0;
+    ~PinnedBuffer() {
+        if (ptr) cudaFreeHost(ptr);
+    }
+    template <class V> V* get(size_t count) {
+        if (cap < count * sizeof(V)) {
+            if (ptr) cudaFreeHost(ptr);
+            ptr = nullptr;
+            cap = 0;
+            check(cudaMallocHost(&ptr, count * sizeof(V)), "pinned staging");
+            cap = count * sizeof(V);
+        }
+        return static_cast<V*>(ptr);
+    }
+};
+
+// CTAs of an extrema launch: four per SM (all resident, 32 warps each SM at
+// 512 threads) as far as every thread has its four vectors.
+constexpr unsigned kExtremaBlocks = 148 * 4;
+
 template <class T>
 static void extrema(const T* d_in, uint64_t n, double* mn, double* mx, cudaStream_t stream) {
     need(d_in && n, "extrema requires at least one element");
-    Carver cv{t_arena.reserve(256)};
-    auto* keys = cv.take<unsigned long long>(2);
-    const unsigned long long init[2] = {~0ull, 0ull};
-    uint64_t* pin = pinned();
-    std::memcpy(pin, init, 16);
-    check(cudaMemcpyAsync(keys, pin, 16, cudaMemcpyHostToDevice, stream), "extrema init");
-    extrema_kernel<T><<<grid_for(n, 256), 256, 0, stream>>>(d_in, n, keys); note_launch();
+    static thread_local PinnedBuffer partial;
+    double* out = partial.get<double>(2 * kExtremaBlocks);
+    const uint64_t per = uint64_t(kExtremaThreads) * 4 * (16 / sizeof(T));
+    const unsigned blocks = unsigned(std::min<uint64_t>((n + per - 1) / per, kExtremaBlocks));
+    extrema_kernel<T><<<blocks, kExtremaThreads, 0, stream>>>(d_in, n, out); note_launch();
     check(cudaGetLastError(), "extrema launch");
-    check(cudaMemcpyAsync(pin + 2, keys, 16, cudaMemcpyDeviceToHost, stream), "extrema readback");
     check(cudaStreamSynchronize(stream), "extrema");
-    auto value = [](unsigned long long k) {
-        const unsigned long long b = (k >> 63) ? (k & 0x7fffffffffffffffull) : ~k;
-        double d;
-        std::memcpy(&d, &b, 8);
-        return d;
-    };
-    *mn = value(pin[2]);
-    *mx = value(pin[3]);
+    double lo = out[0], hi = out[1];
+    for (unsigned b = 1; b < blocks; ++b) {
+        lo = std::fmin(lo, out[2 * b]);
+        hi = std::fmax(hi, out[2 * b + 1]);
+    }
+    *mn = lo;
+    *mx = hi;
 }
 
 // ------------------------------------------------------------ batched compress
@@ -1776,25 +1795,6 @@ static void capture_batch(BatchStreams& bs, int branches, CachedGraph& cg, std::
     cg.device = dev;
     cg.key = std::move(key);
 }
-
-// Pinned host staging that grows on demand.
-struct PinnedBuffer {
-    void* ptr = nullptr;
-    size_t cap = 0;
-    ~PinnedBuffer() {
-        if (ptr) cudaFreeHost(ptr);
-    }
-    template <class V> V* get(size_t count) {
-        if (cap < count * sizeof(V)) {
-            if (ptr) cudaFreeHost(ptr);
-            ptr = nullptr;
-            cap = 0;
-            check(cudaMallocHost(&ptr, count * sizeof(V)), "pinned staging");
-            cap = count * sizeof(V);
-        }
-        return static_cast<V*>(ptr);
-    }
-};
 
 template <class V> static void append_key(std::vector<unsigned char>& key, const V& v) {
     const unsigned char* p = reinterpret_cast<const unsigned char*>(&v);
