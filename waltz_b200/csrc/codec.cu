@@ -186,27 +186,13 @@ static inline Dims halve(Dims d, int mask) {
     return {(mask & AX) ? half_len(d.x) : d.x, (mask & AY) ? half_len(d.y) : d.y, (mask & AZ) ? half_len(d.z) : d.z};
 }
 
-// Tile shapes per schedule (UX, UY, UZ).
-template <class T> struct Tiles;
-template <> struct Tiles<float> {
-    static constexpr int XYZ[3] = {32, 8, 16};
-    static constexpr int XY[3] = {32, 16, 4};
-    static constexpr int Z[3] = {32, 8, 16};
-};
-template <> struct Tiles<double> {
-    static constexpr int XYZ[3] = {16, 8, 8};
-    static constexpr int XY[3] = {32, 16, 4};
-    static constexpr int Z[3] = {32, 8, 8};
-};
-
 // Tuning options of the calling thread (performance only: results do not
 // depend on them; set through waltz_b200_set_option).
 struct Options {
     bool stage_kernels = true; // plane schedule: whole-stage kernels where they fit
     uint32_t zmarch = 0;       // forward z-march planes per CTA: 0 = automatic
-    uint64_t small_level = uint64_t(1) << 15; // inverse levels of at most this many samples: direct staging
-    uint64_t small_fwd = uint64_t(1) << 20;   // forward levels of at most this many samples: direct staging,
-                                              // short z ranges (measured on 128^3 .. 512^3 fields)
+    uint64_t small_level = uint64_t(1) << 15; // inverse levels of at most this many samples: register marches
+    uint64_t small_fwd = uint64_t(1) << 20;   // forward levels of at most this many samples: register marches
     uint32_t repair_scale = 0; // compact repair section (WPW1) with step eb / scale: 0 (off), 16 or 64
     uint32_t xy_march = 0;     // plane schedule: XY levels as the warp march instead of the staged kernels
                                // (bit 0: forward levels, bit 1: inverse levels)
@@ -214,26 +200,6 @@ struct Options {
     uint64_t small_march_fwd = 0; // dyadic forward levels of at most this many samples: XY march + Z march
 };
 static thread_local Options t_opt;
-
-template <class T, bool Inverse, int Mask, int UX, int UY, int UZ, class Src, class Out>
-static void launch_level(const Src& src, Dims a, const Out& out, Sink& sink) {
-    using Op = LevelOp<T, Inverse, Mask, UX, UY, UZ, Src, Out>;
-    constexpr size_t smem = level_smem<T, Inverse, Mask, UX, UY, UZ>();
-    const Dims grid{(a.x + UX - 1) / UX, (a.y + UY - 1) / UY, (a.z + UZ - 1) / UZ};
-    const uint64_t blocks = uint64_t(grid.x) * grid.y * grid.z;
-    need(blocks < (1ull << 31), "Waltz: level grid too large");
-    sink.run<Op>(typename Op::Params{src, a, grid, out}, uint32_t(blocks), smem);
-}
-
-template <class T, bool Inverse, int Mask, class Src, class Out>
-static void level(const Src& src, Dims a, const Out& out, Sink& sink) {
-    if constexpr (Mask == (AX | AY | AZ))
-        launch_level<T, Inverse, Mask, Tiles<T>::XYZ[0], Tiles<T>::XYZ[1], Tiles<T>::XYZ[2]>(src, a, out, sink);
-    else if constexpr (Mask == (AX | AY))
-        launch_level<T, Inverse, Mask, Tiles<T>::XY[0], Tiles<T>::XY[1], Tiles<T>::XY[2]>(src, a, out, sink);
-    else
-        launch_level<T, Inverse, Mask, Tiles<T>::Z[0], Tiles<T>::Z[1], Tiles<T>::Z[2]>(src, a, out, sink);
-}
 
 // One Z level of the plane schedule as a per-column register march
 // (ZMarchOp): a warp per 32 columns and run of windows. A single field's
@@ -290,24 +256,20 @@ template <class K> static uint64_t resident_slots(K kernel, size_t smem, int thr
     return slots;
 }
 
-// One dyadic forward level as a z-march: XY tiles, and the z axis split into
+// One forward level as a z-march: XY tiles, and the z axis split into
 // ranges only as far as needed to give every resident CTA slot work (one
 // range per column tile when many fields share the GPU). Planes are staged by
-// TMA when the source rows meet the copy engine's alignment.
+// TMA; returns false, with nothing launched, when the source rows do not meet
+// the copy engine's alignment.
 template <class T, bool Z, int NT>
-static void level_fwd_stream_nt(const FwdSrc<T>& src, Dims a, const FwdOut<T>& out, uint32_t* status, Sink& sink) {
+static bool level_fwd_stream_nt(const FwdSrc<T>& src, Dims a, const FwdOut<T>& out, uint32_t* status, Sink& sink) {
     constexpr int UX = StreamTile<T>::UX, UY = StreamTile<T>::UY, Q = StreamTile<T>::Q;
     using S = StreamShape<T, UX, UY, Q, NT>;
-    using OpT = FwdStreamOp<T, UX, UY, Q, true, Z, NT>;
-    using OpL = FwdStreamOp<T, UX, UY, Q, false, Z, NT>;
-    typename OpT::Params p{};
-    // small levels: almost every tile is an edge tile, whose reflected cells
-    // the TMA path fixes up one by one; direct staging reflects on load
-    const bool small = vol(a) <= t_opt.small_fwd;
-    const bool tma = !small && make_map_3d<T>(&p.map, src.p, a.x, a.y, a.z, src.sy, src.sz, S::FX, S::FY, 1);
+    using Op = FwdStreamOp<T, UX, UY, Q, Z, NT>;
+    typename Op::Params p{};
+    if (!make_map_3d<T>(&p.map, src.p, a.x, a.y, a.z, src.sy, src.sz, S::FX, S::FY, 1)) return false;
     const uint32_t tx = (a.x + UX - 1) / UX, ty = (a.y + UY - 1) / UY;
     const uint64_t tiles = uint64_t(tx) * ty;
-    const uint32_t min_range = small || !Z ? 8 : 16;
     // planes a z range re-reads besides its own: the z halo of the pipeline
     // (none for an XY level, whose ranges only repeat the CTA's set-up)
     const double reread = Z ? 8.0 : 1.0;
@@ -316,17 +278,17 @@ static void level_fwd_stream_nt(const FwdSrc<T>& src, Dims a, const FwdOut<T>& o
         zrange = std::min(zrange, std::max<uint32_t>(16, t_opt.zmarch + (t_opt.zmarch & 1)));
     } else if (!sink.many) {
         // maximise (filled share of the last wave) x (planes kept out of the
-        // 8-plane halo a range re-reads), over up to 16 ranges of >= 16 planes
-        // (>= 8 for small levels, which are latency-bound)
+        // 8-plane halo a range re-reads), over up to 16 ranges of >= 16
+        // planes (>= 8 for an XY level)
         static thread_local int device = -1;
         static thread_local size_t granted = 0;
-        opt_in_smem(op_kernel_for<OpT>(), S::smem, device, granted);
-        const uint64_t slots = resident_slots(op_kernel_for<OpT>(), S::smem);
+        opt_in_smem(op_kernel_for<Op>(), S::smem, device, granted);
+        const uint64_t slots = resident_slots(op_kernel_for<Op>(), S::smem);
         double best = -1;
         for (uint32_t k = 1; k <= 16; ++k) {
             uint32_t r = (a.z + k - 1) / k;
             r += r & 1;
-            if (k > 1 && r < min_range) break;
+            if (k > 1 && r < (Z ? 16u : 8u)) break;
             const uint64_t blocks = tiles * ((a.z + r - 1) / r);
             const double waves = double((blocks + slots - 1) / slots);
             const double score = double(blocks) / (waves * double(slots)) * double(r) / (double(r) + reread);
@@ -346,48 +308,44 @@ static void level_fwd_stream_nt(const FwdSrc<T>& src, Dims a, const FwdOut<T>& o
     p.zrange = zrange;
     p.out = out;
     p.status = status;
-    if (tma) {
-        sink.run<OpT>(p, uint32_t(blocks), S::smem);
-    } else {
-        typename OpL::Params q{};
-        q.src = src;
-        q.a = a;
-        q.tiles_x = tx;
-        q.tiles_y = ty;
-        q.zrange = zrange;
-        q.out = out;
-        q.status = status;
-        sink.run<OpL>(q, uint32_t(blocks), S::smem);
-    }
+    sink.run<Op>(p, uint32_t(blocks), S::smem);
+    return true;
 }
 
 // Thread count of a z-march CTA: float dyadic levels of one field up to
 // 2^24 samples run 512 threads per CTA, the rest 256.
 template <class T, bool Z = true>
-static void level_fwd_stream(const FwdSrc<T>& src, Dims a, const FwdOut<T>& out, uint32_t* status, Sink& sink) {
+static bool level_fwd_stream(const FwdSrc<T>& src, Dims a, const FwdOut<T>& out, uint32_t* status, Sink& sink) {
     if (sizeof(T) == 4 && Z && !sink.many && !sink.rec && vol(a) <= (uint64_t(1) << 24))
-        level_fwd_stream_nt<T, Z, 512>(src, a, out, status, sink);
-    else
-        level_fwd_stream_nt<T, Z, 256>(src, a, out, status, sink);
+        return level_fwd_stream_nt<T, Z, 512>(src, a, out, status, sink);
+    return level_fwd_stream_nt<T, Z, 256>(src, a, out, status, sink);
 }
 
-// One dyadic inverse level from TMA-staged parity boxes when the coefficient
-// rows meet the copy engine's alignment; the generic level kernel otherwise.
+// One dyadic forward level as two register marches: the Y and X analysis
+// into `tmp` (x/y split, z spatial), then the Z analysis to `out` (the
+// z-march's Y, X, Z order).
+template <class T>
+static void level_fwd_march(const FwdSrc<T>& src, Dims a, const FwdOut<T>& out, T* tmp, Sink& sink) {
+    const size_t ty = a.x, tz = size_t(a.x) * a.y;
+    level_xy<T, false>(src, a, FwdOut<T>{tmp, ty, tz, nullptr, halve(a, AX | AY), a, AX | AY}, sink);
+    level_z<T, false>(FwdSrc<T>{tmp, ty, tz}, a, FwdOut<T>{out.dst, out.sy, out.sz, out.low, out.lo, a, AZ}, sink);
+}
+
+// One dyadic inverse level from TMA-staged parity boxes; returns false, with
+// nothing launched, when the coefficient rows do not meet the copy engine's
+// alignment.
 template <class T, class Out>
-static void level_inv(const InvSrc<T>& src, Dims a, const Out& out, uint32_t* status, Sink& sink) {
+static bool level_inv(const InvSrc<T>& src, Dims a, const Out& out, uint32_t* status, Sink& sink) {
     constexpr int UX = InvTile<T>::UX, UY = InvTile<T>::UY, UZ = InvTile<T>::UZ;
     using S = InvShape<T, UX, UY, UZ>;
     using Op = InvTileOp<T, UX, UY, UZ, Out>;
     typename Op::Params p{};
-    bool tma = vol(a) > t_opt.small_level && half_len(a.x) % S::V == 0 &&
+    bool tma = half_len(a.x) % S::V == 0 &&
                make_map_3d<T>(&p.cmap, src.base, a.x, a.y, a.z, src.sy, src.sz, S::BX, S::HY, S::HZ);
     if (tma && src.low)
         tma = make_map_3d<T>(&p.lmap, src.low, src.lo.x, src.lo.y, src.lo.z, src.lo.x, uint64_t(src.lo.x) * src.lo.y,
                              S::BX, S::HY, S::HZ);
-    if (!tma) {
-        level<T, true, AX | AY | AZ>(src, a, out, sink);
-        return;
-    }
+    if (!tma) return false;
     const uint32_t tx = (a.x + UX - 1) / UX, ty = (a.y + UY - 1) / UY, tz = (a.z + UZ - 1) / UZ;
     const uint64_t blocks = uint64_t(tx) * ty * tz;
     need(blocks < (1ull << 31), "Waltz: level grid too large");
@@ -397,9 +355,10 @@ static void level_inv(const InvSrc<T>& src, Dims a, const Out& out, uint32_t* st
     p.out = out;
     p.status = status;
     sink.run<Op>(p, uint32_t(blocks), S::smem);
+    return true;
 }
 
-// One small dyadic inverse level as two register marches: the Z synthesis
+// One dyadic inverse level as two register marches: the Z synthesis
 // (ZMarchOp, canonical folded windows) into `tmp` in the level's x/y split
 // layout, then the X and Y synthesis (XYMarchOp, canonical Y windows of 8)
 // to `out`. The passes are the tile inverse's Z, X and Y passes, sample for
@@ -411,24 +370,21 @@ static void level_inv_march(const InvSrc<T>& src, Dims a, const Out& out, T* tmp
     level_xy<T, true>(InvSrc<T>{tmp, a.x, size_t(a.x) * a.y, nullptr, Dims{}}, a, out, sink);
 }
 
-// One inverse XY level of the plane schedule from TMA-staged parity boxes
-// when the coefficient rows meet the copy engine's alignment; the generic
-// level kernel otherwise.
+// One inverse XY level of the plane schedule from TMA-staged parity boxes;
+// returns false, with nothing launched, when the coefficient rows do not meet
+// the copy engine's alignment.
 template <class T, class Out>
-static void level_inv_xy(const InvSrc<T>& src, Dims a, const Out& out, uint32_t* status, Sink& sink) {
+static bool level_inv_xy_tiles(const InvSrc<T>& src, Dims a, const Out& out, uint32_t* status, Sink& sink) {
     constexpr int UX = InvTileXY<T>::UX, UY = InvTileXY<T>::UY, UZ = InvTileXY<T>::UZ;
     using S = InvXYShape<T, UX, UY, UZ>;
     using Op = InvTileXYOp<T, UX, UY, UZ, Out>;
     typename Op::Params p{};
-    bool tma = vol(a) > t_opt.small_level && half_len(a.x) % S::V == 0 &&
+    bool tma = half_len(a.x) % S::V == 0 &&
                make_map_3d<T>(&p.cmap, src.base, a.x, a.y, a.z, src.sy, src.sz, S::BX, S::HY, UZ);
     if (tma && src.low)
         tma = make_map_3d<T>(&p.lmap, src.low, src.lo.x, src.lo.y, src.lo.z, src.lo.x, uint64_t(src.lo.x) * src.lo.y,
                              S::BX, S::HY, UZ);
-    if (!tma) {
-        level<T, true, AX | AY>(src, a, out, sink);
-        return;
-    }
+    if (!tma) return false;
     const uint32_t tx = (a.x + UX - 1) / UX, ty = (a.y + UY - 1) / UY, tz = (a.z + UZ - 1) / UZ;
     const uint64_t blocks = uint64_t(tx) * ty * tz;
     need(blocks < (1ull << 31), "Waltz: level grid too large");
@@ -438,6 +394,16 @@ static void level_inv_xy(const InvSrc<T>& src, Dims a, const Out& out, uint32_t*
     p.out = out;
     p.status = status;
     sink.run<Op>(p, uint32_t(blocks), S::smem);
+    return true;
+}
+
+// One inverse XY level of the plane schedule: the warp march where its knob
+// asks for it, on small levels and on rows that the copy engine cannot take
+// (as for the dyadic levels), else the staged tiles.
+template <class T, class Out>
+static void level_inv_xy(const InvSrc<T>& src, Dims a, const Out& out, uint32_t* status, Sink& sink) {
+    if ((t_opt.xy_march & 2u) || vol(a) <= t_opt.small_level || !level_inv_xy_tiles<T>(src, a, out, status, sink))
+        level_xy<T, true>(src, a, out, sink);
 }
 
 // WZP encoder of one magnitude source: one CTA per 8192-sample chunk.
@@ -565,18 +531,14 @@ static void forward(const Geometry& g, const T* in, T* C, T* lowA, T* lowB, T* i
         for (unsigned l = 0; l < g.lxy; ++l) {
             const Dims a = g.dyad[l], lo = halve(a, AX | AY | AZ);
             const bool last = l + 1 == g.lxy;
-            if (vol(a) <= t_opt.small_march_fwd) {
-                // a small level as two marches: the Y and X analysis into
-                // `inter` (x/y split, z spatial), then the Z analysis to C
-                // and the compact low band (the z-march's Y, X, Z order)
-                const size_t isy = a.x, isz = size_t(a.x) * a.y;
-                level_xy<T, false>(src, a, FwdOut<T>{inter, isy, isz, nullptr, halve(a, AX | AY), a, AX | AY}, sink);
-                level_z<T, false>(FwdSrc<T>{inter, isy, isz}, a,
-                                  FwdOut<T>{C, sy, sz, last ? nullptr : lows[l & 1], lo, a, AZ}, sink);
-            } else {
-                FwdOut<T> out{C, sy, sz, last ? nullptr : lows[l & 1], lo, a, AX | AY | AZ};
-                level_fwd_stream<T>(src, a, out, status, sink);
-            }
+            // small levels, and rows that the copy engine cannot take, as two
+            // marches through `inter` (unused by the dyadic schedule): at
+            // 301 x 333 x 325 f32 the finest level takes 0.145 ms so and
+            // took 0.279 with tiles staged by reflecting loads
+            const FwdOut<T> out{C, sy, sz, last ? nullptr : lows[l & 1], lo, a, AX | AY | AZ};
+            if (vol(a) <= std::max(t_opt.small_march_fwd, t_opt.small_fwd) ||
+                !level_fwd_stream<T>(src, a, out, status, sink))
+                level_fwd_march<T>(src, a, out, inter, sink);
             static const char* const kFwdNames[5] = {"fwd_l0", "fwd_l1", "fwd_l2", "fwd_l3", "fwd_l4"};
             sink.mark(kFwdNames[l]);
             src = FwdSrc<T>{lows[l & 1], lo.x, size_t(lo.x) * lo.y};
@@ -609,8 +571,9 @@ static void forward(const Geometry& g, const T* in, T* C, T* lowA, T* lowB, T* i
         const Dims a = g.xyl[l], lo = halve(a, AX | AY);
         const bool last = l + 1 == g.lxy;
         FwdOut<T> out{C, sy, sz, last ? nullptr : lows[l & 1], lo, a, AX | AY};
-        if (t_opt.xy_march & 1u) level_xy<T, false>(src, a, out, sink);
-        else level_fwd_stream<T, false>(src, a, out, status, sink);
+        if ((t_opt.xy_march & 1u) || vol(a) <= t_opt.small_fwd ||
+            !level_fwd_stream<T, false>(src, a, out, status, sink))
+            level_xy<T, false>(src, a, out, sink);
         src = FwdSrc<T>{lows[l & 1], lo.x, size_t(lo.x) * lo.y};
     }
     if (g.lxy) sink.mark("fwd_xy");
@@ -651,20 +614,22 @@ static void inverse(const Geometry& g, T* C, T* bank1, T* bank2, const Final& fi
         for (int l = int(g.lxy) - 1; l >= 0; --l) {
             const Dims a = g.dyad[l];
             InvSrc<T> src{C, sy, sz, low, halve(a, AX | AY | AZ)};
-            // small levels: two marches through bank1 (unused by the dyadic
-            // schedule) instead of the tile inverse
-            const bool march = vol(a) <= t_opt.small_march;
+            // rows that the copy engine cannot take: two marches through
+            // bank1 (unused by the dyadic schedule). At 301 x 333 x 325 the
+            // finest level takes 0.146 ms (f32) so and took 0.590 with tiles
+            // staged by reflecting loads; f64 at 181 x 257 x 333: 0.147 and
+            // 0.479. Small levels take the marches too (their tiles cannot
+            // fill the GPU).
+            const bool march = vol(a) <= std::max(t_opt.small_march, t_opt.small_level);
             if (l > 0) {
                 T* dst = halves[l & 1];
                 const StoreOut<T> to{dst, a.x, size_t(a.x) * a.y};
-                if (march) level_inv_march<T>(src, a, to, bank1, sink);
-                else level_inv<T>(src, a, to, status, sink);
+                if (march || !level_inv(src, a, to, status, sink)) level_inv_march<T>(src, a, to, bank1, sink);
                 low = dst;
                 static const char* const kInvNames[5] = {"inv_l0", "inv_l1", "inv_l2", "inv_l3", "inv_l4"};
                 sink.mark(kInvNames[l]);
             } else {
-                if (march) level_inv_march<T>(src, a, fin, bank1, sink);
-                else level_inv<T>(src, a, fin, status, sink);
+                if (march || !level_inv(src, a, fin, status, sink)) level_inv_march<T>(src, a, fin, bank1, sink);
                 sink.mark(final_stage);
             }
         }
@@ -689,18 +654,15 @@ static void inverse(const Geometry& g, T* C, T* bank1, T* bank2, const Final& fi
             if (l > 0) {
                 T* dst = halves[l & 1];
                 const StoreOut<T> to{dst, a.x, size_t(a.x) * a.y};
-                if (t_opt.xy_march & 2u) level_xy<T, true>(src, a, to, sink);
-                else level_inv_xy<T>(src, a, to, status, sink);
+                level_inv_xy<T>(src, a, to, status, sink);
                 low = dst;
             } else if (g.lz) {
                 const StoreOut<T> to{bank1, sy, sz};
-                if (t_opt.xy_march & 2u) level_xy<T, true>(src, a, to, sink);
-                else level_inv_xy<T>(src, a, to, status, sink);
+                level_inv_xy<T>(src, a, to, status, sink);
                 zbase = bank1;
                 zping[1] = C; // the coefficients are no longer read
             } else {
-                if (t_opt.xy_march & 2u) level_xy<T, true>(src, a, fin, sink);
-                else level_inv_xy<T>(src, a, fin, status, sink);
+                level_inv_xy<T>(src, a, fin, status, sink);
             }
         }
         sink.mark("inv_xy");

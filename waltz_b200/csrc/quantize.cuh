@@ -182,10 +182,10 @@ template <class T> struct CopyFiniteOp {
 // Encoder repair emitter for the finest synthesis: err = T(value - orig);
 // a sample is patched iff |err| > T(eb); the corrected value must be finite
 // and strictly within eb of the original (cpu/src/repair_avx2.cpp:57-74).
-// The original is fetched ahead of the synthesis (kPrefetch). A corrected
-// value whose rounded float difference is at most `safe` (eb shrunk by
-// 2^-21, rounded down) passes the strict double check for certain, so only
-// values near the bound take the two-difference test; float only.
+// The original is fetched ahead of the synthesis (kPrefetch). A value whose
+// rounded difference is at most `safe` (eb shrunk by 2^-21, rounded down)
+// passes the strict double check for certain, so only values near the bound
+// take the two-difference test.
 template <class T> struct RepairOut {
     const T* orig;
     size_t sy, sz;
@@ -194,7 +194,7 @@ template <class T> struct RepairOut {
     uint32_t* pbits;  // row-major bitmap of patched samples
     T* perr;          // dense errors (sparse use)
     uint32_t* status;
-    T safe;           // float: fast-accept threshold; double: unused
+    T safe;           // fast-accept threshold
     static constexpr bool kPrefetch = true;
     __device__ __forceinline__ T fetch(uint32_t x, uint32_t y, uint32_t z) const {
         return __ldg(orig + size_t(z) * sz + size_t(y) * sy + x);
@@ -203,18 +203,16 @@ template <class T> struct RepairOut {
     __device__ __forceinline__ void warm(uint32_t x, uint32_t y, uint32_t z) const {
         asm volatile("prefetch.global.L2 [%0];" ::"l"(orig + size_t(z) * sz + size_t(y) * sy + x));
     }
+    // A rounded error of at most `safe` is below every limit at once: the
+    // sample is not patched, it and its error are finite, and the exact
+    // difference is within the bound. Only the others take the full test.
     __device__ __forceinline__ void emit(uint32_t x, uint32_t y, uint32_t z, T v, T o) const {
         const T err = Lift<T>::sub(v, o);
+        if (fabs(err) <= safe) return;
         const bool patched = fabs(err) > nb;
         const T w = patched ? Lift<T>::sub(v, err) : v;
         bool ok = finite_bits(v) && finite_bits(err) && finite_bits(w);
-        if (ok) {
-            if constexpr (sizeof(T) == 4) {
-                if (!(fabsf(Lift<T>::sub(w, o)) <= safe)) ok = strictly_within(double(w), double(o), bound);
-            } else {
-                ok = strictly_within(double(w), double(o), bound);
-            }
-        }
+        if (ok && !(fabs(Lift<T>::sub(w, o)) <= safe)) ok = strictly_within(double(w), double(o), bound);
         if (patched) {
             const size_t i = size_t(z) * sz + size_t(y) * sy + x;
             atomicOr(&pbits[i >> 5], 1u << (i & 31));

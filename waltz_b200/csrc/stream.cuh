@@ -21,11 +21,11 @@
 //   out: z = 2(j-2) -> e4[j-2] * K, z = 2(j-2)+1 -> o3[j-2] * (-1/K)
 // Outputs are exact from the third pair after the first fed pair on.
 //
-// Staging: with a tensor map the planes arrive as per-plane TMA boxes
-// (FX x FY x 1 at the reflected z), the copy of the next Q planes overlapping
-// the X and Z passes of the current ones; cells of edge tiles that fall
-// outside the array are then reflected in shared memory. Without a map
-// (unaligned rows) the planes are staged with batched ordinary loads.
+// Staging: the planes arrive as per-plane TMA boxes (FX x FY x 1 at the
+// reflected z), the copy of the next Q planes overlapping the X and Z passes
+// of the current ones; cells of edge tiles that fall outside the array are
+// then reflected in shared memory. Levels whose rows do not meet the copy
+// engine's alignment take the register marches instead.
 #pragma once
 #include "common.cuh"
 #include "tma.cuh"
@@ -64,15 +64,14 @@ __device__ __forceinline__ unsigned long long abs_bits(double v) {
 __device__ __forceinline__ bool nonfinite_max(uint32_t m) { return m >= 0x7f800000u; }
 __device__ __forceinline__ bool nonfinite_max(unsigned long long m) { return m >= 0x7ff0000000000000ull; }
 
-// Tma: stage planes with per-plane tensor-map boxes; otherwise with batched
-// ordinary loads. `status` receives ST_WAIT_TIMEOUT if a copy never
-// completes within the wait bound (the block then stops as a whole).
+// `status` receives ST_WAIT_TIMEOUT if a copy never completes within the wait
+// bound (the block then stops as a whole).
 // NT threads per CTA: 256 (four CTAs per SM) for the large levels; 512 (two
 // CTAs per SM, every Y item of a batch of planes in one round) measured
 // faster on the coarser levels, slower on the finest.
-template <class T, int UX, int UY, int Q, bool Tma, bool Z = true, int NT = 256> struct FwdStreamOp {
+template <class T, int UX, int UY, int Q, bool Z = true, int NT = 256> struct FwdStreamOp {
     // 256 threads: four CTAs per SM (64 registers), measured faster than
-    // three with more registers, for both staging forms
+    // three with more registers
     static constexpr int kThreads = NT, kMinBlocks = NT == 512 ? 2 : 4;
     static constexpr bool kGridConstant = true;
     struct Params {
@@ -85,12 +84,12 @@ template <class T, int UX, int UY, int Q, bool Tma, bool Z = true, int NT = 256>
     };
     static __device__ __forceinline__ void run(const Params& P, uint32_t block, uint32_t);
     static __device__ __forceinline__ void acquire_maps(const Params& P) {
-        if (Tma) tensormap_acquire(&P.map);
+        tensormap_acquire(&P.map);
     }
 };
 
-template <class T, int UX, int UY, int Q, bool Tma, bool Z, int NT>
-__device__ __forceinline__ void FwdStreamOp<T, UX, UY, Q, Tma, Z, NT>::run(const Params& P, uint32_t block, uint32_t) {
+template <class T, int UX, int UY, int Q, bool Z, int NT>
+__device__ __forceinline__ void FwdStreamOp<T, UX, UY, Q, Z, NT>::run(const Params& P, uint32_t block, uint32_t) {
     const FwdSrc<T> src = P.src;
     const Dims a = P.a;
     const uint32_t tiles_x = P.tiles_x, tiles_y = P.tiles_y, zrange = P.zrange;
@@ -104,7 +103,7 @@ __device__ __forceinline__ void FwdStreamOp<T, UX, UY, Q, Tma, Z, NT>::run(const
     T* In = reinterpret_cast<T*>(stream_smem + ((128 - (smem_u32(stream_smem) & 127)) & 127)); // [Q][FY][FX]
     T* Mid = In + S::IN;                                                                  // [Q][UY][YP]
     uint64_t* bar = reinterpret_cast<uint64_t*>(Mid + S::MID);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5;
     const uint32_t bx = block % tiles_x, by = (block / tiles_x) % tiles_y;
     const uint32_t bzr = block / (tiles_x * tiles_y);
     const uint32_t ox = bx * UX, oy = by * UY;
@@ -145,17 +144,15 @@ __device__ __forceinline__ void FwdStreamOp<T, UX, UY, Q, Tma, Z, NT>::run(const
             tma_load_3d(In + q * S::FY * S::FX, map, int(ox) - 4, int(oy) - 4, int(mirror(zb + q, a.z)), bar);
     };
     uint32_t phase = 0;
-    if constexpr (Tma) {
-        if (tid == 0) {
-            mbar_init(bar, 1);
-            fence_barrier_init();
-        }
-        __syncthreads();
-        if (tid == 0) issue(zin0);
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        fence_barrier_init();
     }
+    __syncthreads();
+    if (tid == 0) issue(zin0);
 
     for (int64_t zb = zin0; zb < zin1; zb += Q) {
-        if constexpr (Tma) {
+        {
             // warp 0 polls the barrier; the other warps park at the block
             // barrier instead of spinning on issue slots
             const bool ok = __syncthreads_and(warp != 0 || mbar_wait(bar, phase, kWaitBound));
@@ -198,37 +195,6 @@ __device__ __forceinline__ void FwdStreamOp<T, UX, UY, Q, Tma, Z, NT>::run(const
                 fence_proxy_async(); // these writes precede the next copy into In
                 __syncthreads();
             }
-        } else {
-            // ---- stage Q planes x FY rows of FX samples (reflected)
-            constexpr int ROWS = Q * S::FY;
-            constexpr int kBatch = 6;
-            const uint32_t x0 = mirror(int64_t(ox) + lane - 4, a.x), x1 = mirror(int64_t(ox) + lane + 28, a.x);
-            const bool has0 = lane < S::FX, has1 = lane + 32 < S::FX;
-            for (int r0 = warp; r0 < ROWS; r0 += (NT / 32) * kBatch) {
-                T v0[kBatch], v1[kBatch];
-#pragma unroll
-                for (int u = 0; u < kBatch; ++u) {
-                    const int r = r0 + u * (NT / 32);
-                    v0[u] = T(0);
-                    v1[u] = T(0);
-                    if (r < ROWS) {
-                        const int q = r / S::FY, fy = r % S::FY;
-                        const auto row = src.row(mirror(int64_t(oy) + fy - 4, a.y), mirror(zb + q, a.z));
-                        if (has0) v0[u] = src.get(row, x0);
-                        if (has1) v1[u] = src.get(row, x1);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < kBatch; ++u) {
-                    const int r = r0 + u * (NT / 32);
-                    if (r < ROWS) {
-                        T* dst = In + r * S::FX;
-                        if (has0) dst[lane] = v0[u];
-                        if (has1) dst[lane + 32] = v1[u];
-                    }
-                }
-            }
-            __syncthreads();
         }
         // ---- Y: one window of UY outputs per (plane, column); every staged
         // sample is read here exactly once, so the finiteness check rides along
@@ -257,9 +223,7 @@ __device__ __forceinline__ void FwdStreamOp<T, UX, UY, Q, Tma, Z, NT>::run(const
             }
         }
         __syncthreads();
-        if constexpr (Tma) {
-            if (tid == 0 && zb + Q < zin1) issue(zb + Q); // In is free: overlap the next copy
-        }
+        if (tid == 0 && zb + Q < zin1) issue(zb + Q); // In is free: overlap the next copy
         // ---- X: windows of 16 outputs per (plane, row), in place in Mid
         {
             constexpr int WX = 16, P = WX / 2 + 4, WIN = UX / WX;

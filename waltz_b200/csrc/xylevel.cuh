@@ -68,6 +68,14 @@ template <class T> __device__ __forceinline__ void pair_inverse(T& e, T& o) {
     pair_odd(o, e, -K97<T>::a);
 }
 
+// Emitters that fetch an operand of their own ahead of the value (kPrefetch).
+template <class Out, class = void> struct Prefetching {
+    static constexpr bool value = false;
+};
+template <class Out> struct Prefetching<Out, decltype(void(Out::kPrefetch))> {
+    static constexpr bool value = Out::kPrefetch;
+};
+
 template <class T, bool Inverse, class Src, class Out> struct XYMarchOp {
     static constexpr int kThreads = 256, kMinBlocks = 0; // no occupancy floor: about 80 registers, three CTAs per SM
     struct Params {
@@ -208,6 +216,17 @@ __device__ __forceinline__ void XYMarchOp<T, Inverse, Src, Out>::run(const Param
             ko[j][0] = o[PP - KEEP + j][0], ko[j][1] = o[PP - KEEP + j][1];
         }
         const uint32_t y0 = w * W;
+        // the emitter's own operands (the originals, for repairs): all in
+        // flight before the lifting that hides their latency
+        constexpr bool kPre = Inverse && Prefetching<Out>::value;
+        T pre[kPre ? W : 1][2];
+        if constexpr (kPre) {
+#pragma unroll
+            for (int k = 0; k < W; ++k) {
+                pre[k][0] = (live_e && y0 + k < a.y) ? out.fetch(uint32_t(xe), y0 + k, z) : T(0);
+                pre[k][1] = (live_o && y0 + k < a.y) ? out.fetch(uint32_t(xe) + 1, y0 + k, z) : T(0);
+            }
+        }
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
             // one column of the pair along Y, in registers
@@ -253,6 +272,16 @@ __device__ __forceinline__ void XYMarchOp<T, Inverse, Src, Out>::run(const Param
                 if (y + 1 < a.y) {
                     if (live_e) ro[0] = o[j][0];
                     if (live_o) ro[1] = o[j][1];
+                }
+            } else if constexpr (kPre) {
+                const int k = 2 * (j - 2);
+                if (y < a.y) {
+                    if (live_e) out.emit(x, y, z, e[j][0], pre[k][0]);
+                    if (live_o) out.emit(x + 1, y, z, e[j][1], pre[k][1]);
+                }
+                if (y + 1 < a.y) {
+                    if (live_e) out.emit(x, y + 1, z, o[j][0], pre[k + 1][0]);
+                    if (live_o) out.emit(x + 1, y + 1, z, o[j][1], pre[k + 1][1]);
                 }
             } else {
                 if (y < a.y) {
