@@ -1,10 +1,37 @@
-"""The extrema reduction on the GPU."""
+"""Level kernels at the sizes where their tiles and windows end, and the
+extrema reduction, on the GPU."""
 from __future__ import annotations
 
 import numpy as np
 import pytest
 
+from oracle import oracle as O
+from tests import patterns as P
+from tests.test_gpu_parity import gpu_compress, gpu_decompress, gpu_transform
+
 pytestmark = pytest.mark.gpu
+
+# (nx, ny, nz), dyadic. Strips of 32 x start at 4 mod 32, Z windows hold 16
+# planes, Y windows 8 rows; the finest level's half row is a multiple of 4
+# (the staged kernels) except in the last two (the register marches).
+LEVEL_SHAPES = [(24, 9, 9), (40, 15, 16), (24, 17, 15), (72, 31, 17), (32, 40, 23), (136, 33, 34), (64, 65, 66),
+                (37, 33, 35), (66, 47, 41)]
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("nxyz", LEVEL_SHAPES)
+def test_levels_bit_exact_at_their_edges(nxyz, dtype):
+    rng = np.random.default_rng(sum(nxyz))
+    a = rng.standard_normal(P.zyx(nxyz)).astype(dtype)
+    f = gpu_transform(a, inverse=False)
+    assert f.tobytes() == O.transform(a, inverse=False).tobytes()
+    assert gpu_transform(f, inverse=True).tobytes() == O.transform(f, inverse=True).tobytes()
+    # 1e-1 on noise leaves many samples to repair, 1e-4 few
+    for eb in (float(np.float32(1e-1)), float(np.float32(1e-4))):
+        expect = O.compress(a, eb)
+        assert gpu_compress(a, eb) == expect
+        assert gpu_decompress(expect, a.shape, dtype).tobytes() == O.decompress(expect, a.shape, dtype).tobytes()
+
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("n", [1, 2, 5, 31, 511, 8191, 8193, 3_000_001])

@@ -12,6 +12,7 @@
 #include "common.cuh"
 #include "compact.cuh"
 #include "inverse.cuh"
+#include "invmarch.cuh"
 #include "launch.cuh"
 #include "ops.cuh"
 #include "quantize.cuh"
@@ -331,11 +332,58 @@ static void level_fwd_march(const FwdSrc<T>& src, Dims a, const FwdOut<T>& out, 
     level_z<T, false>(FwdSrc<T>{tmp, ty, tz}, a, FwdOut<T>{out.dst, out.sy, out.sz, out.low, out.lo, a, AZ}, sink);
 }
 
-// One dyadic inverse level from TMA-staged parity boxes; returns false, with
+// One dyadic inverse level from TMA-staged parity boxes (float: the y-march
+// of invmarch.cuh; double: the tiles of inverse.cuh); returns false, with
 // nothing launched, when the coefficient rows do not meet the copy engine's
 // alignment.
-template <class T, class Out>
-static bool level_inv(const InvSrc<T>& src, Dims a, const Out& out, uint32_t* status, Sink& sink) {
+template <class Out>
+static bool level_inv(const InvSrc<float>& src, Dims a, const Out& out, uint32_t* status, Sink& sink) {
+    using S = InvMarch;
+    using Op = InvMarchOp<Out>;
+    typename Op::Params p{};
+    bool tma = half_len(a.x) % 4 == 0 &&
+               make_map_3d<float>(&p.cmap, src.base, a.x, a.y, a.z, src.sy, src.sz, S::HX, S::HY, S::HZ);
+    if (tma && src.low)
+        tma = make_map_3d<float>(&p.lmap, src.low, src.lo.x, src.lo.y, src.lo.z, src.lo.x,
+                                 uint64_t(src.lo.x) * src.lo.y, S::HX, S::HY, S::HZ);
+    if (!tma) return false;
+    const uint32_t wins = (a.y + S::UY - 1) / S::UY;
+    p.strips = (a.x + S::SHIFT + S::UX - 1) / S::UX;
+    p.zwins = (a.z + S::UZ - 1) / S::UZ;
+    const uint64_t columns = uint64_t(p.strips) * p.zwins;
+    // Y windows per CTA: whole columns when many fields fill the GPU; for one
+    // field the split with the fewest steps along its waves of resident CTAs,
+    // a CTA's priming step counted as two thirds of a window (512^3 repair
+    // level: 0.453 ms at 16 windows a CTA, 0.493 at 3, 0.590 at all 64)
+    p.seg = wins;
+    if (!sink.many) {
+        static thread_local int device = -1;
+        static thread_local size_t granted = 0;
+        opt_in_smem(op_kernel_for<Op>(), S::smem, device, granted);
+        const uint64_t slots = resident_slots(op_kernel_for<Op>(), S::smem);
+        double best = 0;
+        for (uint32_t k = 1; k <= 32 && k <= wins; ++k) {
+            const uint32_t seg = (wins + k - 1) / k;
+            const uint64_t blocks = columns * ((wins + seg - 1) / seg);
+            const double steps = double((blocks + slots - 1) / slots) * (seg + 0.67);
+            if (k == 1 || steps < best) {
+                best = steps;
+                p.seg = seg;
+            }
+        }
+    }
+    const uint64_t blocks = columns * ((wins + p.seg - 1) / p.seg);
+    need(blocks < (1ull << 31), "Waltz: level grid too large");
+    p.lv = InvLevel<float>{src.base, src.sy, src.sz, src.low, src.lo, a};
+    p.out = out;
+    p.status = status;
+    sink.run<Op>(p, uint32_t(blocks), S::smem);
+    return true;
+}
+
+template <class Out>
+static bool level_inv(const InvSrc<double>& src, Dims a, const Out& out, uint32_t* status, Sink& sink) {
+    using T = double;
     constexpr int UX = InvTile<T>::UX, UY = InvTile<T>::UY, UZ = InvTile<T>::UZ;
     using S = InvShape<T, UX, UY, UZ>;
     using Op = InvTileOp<T, UX, UY, UZ, Out>;
@@ -618,9 +666,10 @@ static void inverse(const Geometry& g, T* C, T* bank1, T* bank2, const Final& fi
             // bank1 (unused by the dyadic schedule). At 301 x 333 x 325 the
             // finest level takes 0.146 ms (f32) so and took 0.590 with tiles
             // staged by reflecting loads; f64 at 181 x 257 x 333: 0.147 and
-            // 0.479. Small levels take the marches too (their tiles cannot
-            // fill the GPU).
-            const bool march = vol(a) <= std::max(t_opt.small_march, t_opt.small_level);
+            // 0.479. Small double levels take the marches too (their tiles
+            // cannot fill the GPU); the float y-march was at least as fast as
+            // two marches on every level measured (16^3 to 512^3 samples).
+            const bool march = sizeof(T) == 8 && vol(a) <= std::max(t_opt.small_march, t_opt.small_level);
             if (l > 0) {
                 T* dst = halves[l & 1];
                 const StoreOut<T> to{dst, a.x, size_t(a.x) * a.y};

@@ -220,6 +220,31 @@ template <class T> struct RepairOut {
         }
         if (!ok) atomicOr(status, ST_BOUND);
     }
+    // Whole-warp form for lanes that hold consecutive x of one row, sample i
+    // of the field in this lane (`live`: inside it). Returns the row's mask of
+    // patched lanes; the caller hands it to put_row.
+    __device__ __forceinline__ uint32_t emit_row(T v, T o, size_t i, bool live) const {
+        const T err = Lift<T>::sub(v, o);
+        const bool full = live && !(fabs(err) <= safe);
+        if (!__any_sync(0xffffffffu, full)) return 0u;
+        const bool patched = full && fabs(err) > nb;
+        if (patched) perr[i] = err;
+        // patched and within `safe` of the original: finite and in the bound
+        if (full && !(patched && fabs(Lift<T>::sub(Lift<T>::sub(v, err), o)) <= safe)) check_full(v, o, err, patched);
+        return __ballot_sync(0xffffffffu, patched);
+    }
+    __device__ __noinline__ void check_full(T v, T o, T err, bool patched) const {
+        const T w = patched ? Lift<T>::sub(v, err) : v;
+        if (!finite_bits(v) || !finite_bits(err) || !finite_bits(w) || !strictly_within(double(w), double(o), bound))
+            atomicOr(status, ST_BOUND);
+    }
+    // Sets the bits of `mask` for the samples i .. i + 31 (i may lie below the
+    // field where the mask's low bits are zero).
+    __device__ __forceinline__ void put_row(int64_t i, uint32_t mask) const {
+        const uint32_t sh = uint32_t(i) & 31u, lo = mask << sh, hi = sh ? mask >> (32 - sh) : 0u;
+        if (lo) atomicOr(&pbits[i >> 5], lo);
+        if (hi) atomicOr(&pbits[(i >> 5) + 1], hi);
+    }
     __device__ __forceinline__ void operator()(uint32_t x, uint32_t y, uint32_t z, T v) const {
         emit(x, y, z, v, fetch(x, y, z));
     }
