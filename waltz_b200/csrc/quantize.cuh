@@ -631,8 +631,8 @@ __global__ void __launch_bounds__(kExtremaThreads) extrema_kernel(const T* __res
     for (; i < nv; i += step) take_vec(vec[i]);
 #pragma unroll
     for (int d = 16; d; d >>= 1) {
-        take(__shfl_xor_sync(0xffffffffu, lo, d));
-        take(__shfl_xor_sync(0xffffffffu, hi, d));
+        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, d));
+        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, d));
     }
     if ((threadIdx.x & 31) == 0) {
         slo[threadIdx.x / 32] = lo;
