@@ -1251,7 +1251,9 @@ template <class T> struct CompressJob {
             if (fused) {
                 uint32_t lb = 0;
                 while ((1u << lb) < bsz) ++lb;
-                launch_wzp_encode(wa, QuantBricks<T>{P.C, nx, ny, g.bz, lb, rank, q, inv, P.qbits, P.qval, P.status},
+                launch_wzp_encode(wa,
+                                  QuantBricks<T>{P.C, nx, ny, g.bz, lb, reciprocal(nx / 16), reciprocal(ny / 16), q,
+                                                 inv, P.qbits, P.qval, P.status},
                                   chunks, sink);
             } else {
                 launch_wzp_encode(wa, MagArrays{P.mag, P.sign}, chunks, sink);

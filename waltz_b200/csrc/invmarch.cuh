@@ -28,36 +28,11 @@
 #pragma once
 #include "common.cuh"
 #include "inverse.cuh"
+#include "packed.cuh"
 #include "quantize.cuh"
 #include "tma.cuh"
 
 namespace wb {
-
-// Two floats in one 64-bit register pair.
-using f2 = unsigned long long;
-__device__ __forceinline__ f2 f2_pack(float lo, float hi) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void f2_unpack(f2 v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
-    f2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 
 // lift_inverse<float, P, true> (common.cuh) on two lines at once.
 template <int P> __device__ __forceinline__ void lift_inverse2(f2 (&e)[P], f2 (&o)[P]) {

@@ -36,6 +36,22 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* tmp, u
     return tmp[warp] + inc - v;
 }
 
+// The same scan with one barrier: every warp folds the warp totals itself.
+// `tmp` must hold NT / 32 words that no earlier scan of the block has used
+// since the last barrier, and stays readable until the next one.
+template <int NT>
+__device__ __forceinline__ uint32_t block_excl_scan1(uint32_t v, uint32_t* tmp, uint32_t& total) {
+    static_assert(NT % 32 == 0 && NT <= 1024, "block size");
+    constexpr int NW = NT / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t inc = warp_incl_scan(v);
+    if (lane == 31) tmp[warp] = inc;
+    __syncthreads();
+    const uint32_t w = lane < NW ? tmp[lane] : 0u;
+    total = __reduce_add_sync(0xffffffffu, w);
+    return __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u) + inc - v;
+}
+
 template <int NT>
 __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* tmp) {
     uint32_t total;

@@ -16,6 +16,7 @@
 // Morton scatter into the row-major coefficient array.
 #pragma once
 #include "common.cuh"
+#include "packed.cuh"
 #include "quantize.cuh"
 #include "scan.cuh"
 
@@ -110,19 +111,16 @@ __device__ __forceinline__ void planes_repack(uint8_t* buf, uint32_t blocks, boo
 
 struct WzpEncodeSmem {
     uint16_t m[kChunk + 8];            // magnitudes (+ slack for word-wide copies)
-    union {
-        uint8_t planes[kEncBytes];     // bit planes, then the eliminated payload in place
-        uint8_t sneg[kChunk];          // negative-code flags while a source quantises
-    };
+    uint8_t planes[kEncBytes];         // bit planes, then the eliminated payload in place
     uint8_t lv[2048 + 256 + 32 + 4 + 4]; // nonzero bitmap and its reductions
     uint32_t sgn[kChunk / 32 + 1];     // compacted sign bits (+ slack)
     uint32_t gcount[kChunk / 32];      // nonzero magnitudes per 32-group
     uint32_t gsign[kChunk / 32];       // per 32-group: sign bits of its nonzero magnitudes, compacted
     uint32_t nsign[kChunk / 32];       // natural sign words of the chunk
-    uint32_t bbase[32];                // row-major bases of the chunk's bricks (quantising source)
     uint32_t sel[16];                  // byte_perm selectors: compact the bytes of a 4-bit mask
-    uint32_t tmp[40];
-    uint32_t chunk, excl;
+    uint8_t pack[256];                 // compressed nibbles: entry 16 * mask + value
+    uint32_t tmp[2][kWzpThreads / 32]; // totals of the two block scans
+    uint32_t chunk, excl, mbytes, raw;
 };
 
 struct WzpEncodeArgs {
@@ -155,12 +153,26 @@ __device__ __forceinline__ uint32_t warp_transpose32(uint32_t x, int lane) {
     return x;
 }
 
+// Bit 7 of every byte of the result: the byte of w is not zero (other bits 0).
+__device__ __forceinline__ uint32_t nonzero_bytes(uint32_t w) {
+    return (((w & 0x7f7f7f7fu) + 0x7f7f7f7fu) | w) & 0x80808080u;
+}
+// Four such flags in the top nibble of a product (the sixteen partial
+// products have distinct places, so nothing carries into bits 28..31).
+constexpr uint32_t kGatherNibble = 0x00204081u;
 // 4-bit mask of the nonzero bytes of w (bit k = byte k).
-__device__ __forceinline__ uint32_t nonzero_nibble(uint32_t w) { return (__vsetne4(w, 0u) * 0x01020408u) >> 24; }
+__device__ __forceinline__ uint32_t nonzero_nibble(uint32_t w) { return (nonzero_bytes(w) * kGatherNibble) >> 28; }
 // 4-bit mask of the bytes of w that differ from the byte before them
 // (`prev` is the byte preceding w).
 __device__ __forceinline__ uint32_t changed_nibble(uint32_t w, uint32_t prev) {
-    return (__vsetne4(w, (w << 8) | (prev & 0xffu)) * 0x01020408u) >> 24;
+    return nonzero_nibble(w ^ ((w << 8) | (prev & 0xffu)));
+}
+// 32-bit mask of the nonzero bytes of eight words.
+__device__ __forceinline__ uint32_t nonzero_mask(const uint32_t (&w)[8]) {
+    uint32_t bits = 0;
+#pragma unroll
+    for (int k = 7; k >= 0; --k) bits = __funnelshift_l(nonzero_bytes(w[k]) * kGatherNibble, bits, 4);
+    return bits;
 }
 // Appends the bytes of w selected by the 4-bit mask to dst + o; returns how many.
 __device__ __forceinline__ uint32_t put_selected(uint8_t* dst, uint32_t o, uint32_t w, uint32_t mask,
@@ -282,51 +294,51 @@ __device__ __forceinline__ void block_origin(uint32_t k, uint32_t zb, uint32_t& 
     }
 }
 
-// Bits of x selected by mask, packed towards bit 0 in order (16-bit
-// compress, Hacker's Delight 7-4).
-__device__ __forceinline__ uint32_t compress16(uint32_t x, uint32_t m) {
-    x &= m;
-    uint32_t mk = (~m << 1) & 0xffffu;
+// Bit compress and expand of 16 bits by nibbles through 256-entry tables in
+// shared memory: about 30 instructions where the shift network of a general
+// 16-bit compress takes 85. Entry 16 m + x of `pack` holds the bits of x
+// selected by m, moved to bit 0 in order; of `spread`, the low popc(m) bits of
+// x moved to the set positions of m.
+__device__ __forceinline__ uint32_t pack_entry(uint32_t i) {
+    const uint32_t m = i >> 4, x = i & 15u;
+    uint32_t v = 0, n = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        uint32_t mp = mk ^ (mk << 1);
-        mp ^= mp << 2;
-        mp ^= mp << 4;
-        mp ^= mp << 8;
-        mp &= 0xffffu;
-        const uint32_t mv = mp & m;
-        m = (m ^ mv) | (mv >> (1 << i));
-        const uint32_t t = x & mv;
-        x = (x ^ t) | (t >> (1 << i));
-        mk &= ~mp;
-    }
-    return x;
+    for (int b = 0; b < 4; ++b)
+        if ((m >> b) & 1u) v |= ((x >> b) & 1u) << n++;
+    return v;
+}
+__device__ __forceinline__ uint32_t spread_entry(uint32_t i) {
+    const uint32_t m = i >> 4, x = i & 15u;
+    uint32_t v = 0, n = 0;
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+        if ((m >> b) & 1u) v |= ((x >> n++) & 1u) << b;
+    return v;
+}
+// The nibbles of a 16-bit value in the low halves of four bytes.
+__device__ __forceinline__ uint32_t nibble_bytes(uint32_t x) {
+    x = (x | (x << 8)) & 0x00ff00ffu;
+    return (x | (x << 4)) & 0x0f0f0f0fu;
+}
+// Bits of x selected by m, packed towards bit 0 in order.
+__device__ __forceinline__ uint32_t compress16(uint32_t x, uint32_t m, const uint8_t* pack) {
+    const uint32_t i = nibble_bytes(x) | (nibble_bytes(m) << 4);
+    return uint32_t(pack[i & 0xffu]) | (uint32_t(pack[(i >> 8) & 0xffu]) << __popc(m & 0xfu)) |
+           (uint32_t(pack[(i >> 16) & 0xffu]) << __popc(m & 0xffu)) | (uint32_t(pack[i >> 24]) << __popc(m & 0xfffu));
+}
+// The low popc(m) bits of x moved to the set positions of m, in order.
+__device__ __forceinline__ uint32_t expand16(uint32_t x, uint32_t m, const uint8_t* spread) {
+    const uint32_t h = nibble_bytes(m) << 4;
+    return uint32_t(spread[(h & 0xf0u) | (x & 15u)]) |
+           (uint32_t(spread[((h >> 8) & 0xf0u) | ((x >> __popc(m & 0xfu)) & 15u)]) << 4) |
+           (uint32_t(spread[((h >> 16) & 0xf0u) | ((x >> __popc(m & 0xffu)) & 15u)]) << 8) |
+           (uint32_t(spread[(h >> 24) | ((x >> __popc(m & 0xfffu)) & 15u)]) << 12);
 }
 
-// The low popc(m) bits of x spread to the set positions of m, in order
-// (16-bit expand, the inverse of compress16).
-__device__ __forceinline__ uint32_t expand16(uint32_t x, uint32_t m) {
-    uint32_t a[4];
-    const uint32_t m0 = m;
-    uint32_t mk = (~m << 1) & 0xffffu;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        uint32_t mp = mk ^ (mk << 1);
-        mp ^= mp << 2;
-        mp ^= mp << 4;
-        mp ^= mp << 8;
-        mp &= 0xffffu;
-        const uint32_t mv = mp & m;
-        a[i] = mv;
-        m = (m ^ mv) | (mv >> (1 << i));
-        mk &= ~mp;
-    }
-#pragma unroll
-    for (int i = 3; i >= 0; --i) {
-        const uint32_t mv = a[i], t = x << (1 << i);
-        x = (x & ~mv) | (t & mv);
-    }
-    return x & m0;
+// Nonzero mask (bit j = magnitude j) of a block from its 16 bit planes.
+__device__ __forceinline__ uint32_t planes_nonzero(const uint32_t (&w)[8]) {
+    const uint32_t z = (w[0] | w[1] | w[2]) | (w[3] | w[4] | w[5]) | (w[6] | w[7]); // bit 15 - j = magnitude j
+    return __brev((z | (z >> 16)) & 0xffffu) >> 16;
 }
 
 // Magnitude sources of the encoder. Each fills S.m[0, 8192) (zeros past
@@ -349,6 +361,52 @@ struct MagArrays {
     }
 };
 
+// Codes of four samples in the short form: one add of 1.5 * 2^(mantissa
+// bits) rounds the scaled value to the nearest integer, ties to even, and the
+// sum's bits less the constant's are that integer (as FastRound, without its
+// range test). `top` collects the largest |code| as an unsigned value and ends
+// above 65535 when a code does not fit 16 bits or its value is outside the
+// rounding's range or not finite; the values are then not to be used. v
+// receives the dequantised values. Codes of zero give +0, as x - x = +0.
+template <class T> struct QuantFast;
+template <> struct QuantFast<float> {
+    static __device__ __forceinline__ void row(float (&v)[4], float inv, float q, int32_t (&c)[4], uint32_t& top) {
+        const f2 q2 = f2_pack(q, q), down = f2_pack(-12582912.0f, -12582912.0f);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            // scalar: a packed product and sum would be contracted (f2_mul)
+            const float t0 = __fadd_rn(__fmul_rn(v[2 * h], inv), 12582912.0f),
+                        t1 = __fadd_rn(__fmul_rn(v[2 * h + 1], inv), 12582912.0f);
+            // an out-of-range sum leaves the constant's binade, so its bits
+            // differ by more than 2^22; the caller's maximum sees that
+            c[2 * h] = int32_t(__float_as_uint(t0) - 0x4b400000u);
+            c[2 * h + 1] = int32_t(__float_as_uint(t1) - 0x4b400000u);
+            f2_unpack(f2_mul(f2_add(f2_pack(t0, t1), down), q2), v[2 * h], v[2 * h + 1]);
+        }
+        (void)top;
+    }
+};
+template <> struct QuantFast<double> {
+    static __device__ __forceinline__ void row(double (&v)[4], double inv, double q, int32_t (&c)[4], uint32_t& top) {
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const double t = __dadd_rn(__dmul_rn(v[x], inv), 6755399441055744.0); // 1.5 * 2^52
+            c[x] = __double2loint(t);
+            // the code fits 32 bits if the high word is the constant's, less
+            // one for a negative code
+            if (uint32_t(__double2hiint(t)) - uint32_t(c[x] >> 31) != 0x43380000u) top = 0xffffffffu;
+            v[x] = __dmul_rn(__dsub_rn(t, 6755399441055744.0), q);
+        }
+    }
+};
+
+// Division by a divisor known to the host: r = reciprocal(d) = floor(2^64 / d)
+// + 1 gives floor(x / d) for every 32-bit x and d > 1; d = 1 has r = 0.
+inline uint64_t reciprocal(uint32_t d) { return d > 1 ? ~uint64_t(0) / d + 1 : 0; }
+__device__ __forceinline__ uint32_t divide(uint32_t x, uint64_t r, uint32_t d) {
+    return d > 1 ? uint32_t(__umul64hi(uint64_t(x), r)) : x;
+}
+
 // The coefficients themselves, quantised by the encoder (quantize_kernel
 // fused in): the chunk is a run of whole 16 x 16 x bz bricks (2^lb samples
 // each, the field made of whole bricks only); every brick is read and
@@ -358,55 +416,84 @@ template <class T> struct QuantBricks {
     static constexpr bool kBlockPlanes = true;
     T* coeff;
     uint32_t nx, ny, bz, lb;
-    const uint16_t* rank; // full-brick slot: brick-local row-major index -> rank
+    uint64_t rnbx, rnby;  // reciprocals of nx / 16 and ny / 16 (reciprocal())
     T q, inv;
     uint32_t* qbits;
     uint32_t* qval;
     uint32_t* status;
 
     // Quantises block t of the chunk starting at `first` (its dequantised
-    // values written back): packed magnitudes w (pairs of Morton slots),
-    // nonzero and negative masks (bit j = slot j of the block).
+    // values written back): packed magnitudes w (pairs of Morton slots) and
+    // the negative mask (bit j = slot j of the block). Rows whose codes fit 16
+    // bits take the short form (QuantFast); the others row_full().
     template <bool Tall>
-    __device__ __forceinline__ void quantise_block(uint32_t first, uint32_t t, uint32_t (&w)[8], uint32_t& zm,
-                                                   uint32_t& nm) const {
+    __device__ __forceinline__ void quantise_block(uint32_t first, uint32_t t, uint32_t (&w)[8], uint32_t& nm) const {
         using Sh = BlockShape<Tall>;
         const uint32_t plane = nx * ny;
         const uint32_t b = (first >> lb) + ((t << 4) >> lb), k = t & ((1u << (lb - 4)) - 1u);
         const uint32_t nbx = nx / 16, nby = ny / 16;
-        const uint32_t bxi = b % nbx, tb = b / nbx, byi = tb % nby, slab = tb / nby;
+        const uint32_t tb = divide(b, rnbx, nbx), bxi = b - tb * nbx, slab = divide(tb, rnby, nby), byi = tb - slab * nby;
         uint32_t lx, ly, lz;
         block_origin(k, lb - 8, lx, ly, lz);
         const uint32_t at0 = (slab * bz + lz) * plane + (byi * 16 + ly) * nx + bxi * 16 + lx;
-        uint32_t bad = 0;
+        constexpr int dd = Sh::d;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            const uint32_t at = at0 + Sh::row_offset(r, nx, plane);
-            constexpr int dd = Sh::d;
             const int e0 = Sh::e0(r), e1 = e0 + dd;
+            T* row = coeff + at0 + Sh::row_offset(r, nx, plane);
             T v[4];
-            load4(coeff + at, v);
-            uint32_t mg[4];
+            load4(row, v);
+            int32_t c[4];
+            uint32_t top = 0;
+            QuantFast<T>::row(v, inv, q, c, top);
+            uint32_t neg = 0; // bit x = sign of sample x
+#pragma unroll
+            for (int x = 3; x >= 0; --x) neg = __funnelshift_l(uint32_t(c[x]), neg, 1);
+            uint32_t m[4];
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
-                int32_t m;
-                bool neg;
-                v[x] = quantize_one<T>(v[x], inv, q, m, neg, bad);
-                const int e = (x < 2 ? e0 : e1) + (x & 1);
-                mg[x] = uint32_t(m > 65535 ? 65535 : m);
-                zm |= uint32_t(m != 0) << e;
-                nm |= uint32_t(neg && m) << e;
-                if (m > 65535) {
-                    atomicOr(&qbits[(at + x) >> 5], 1u << ((at + x) & 31));
-                    qval[at + x] = uint32_t(m);
-                }
+                m[x] = c[x] < 0 ? 0u - uint32_t(c[x]) : uint32_t(c[x]);
+                top = max(top, m[x]);
             }
-            store4(coeff + at, v);
             // e0 and e1 are even: each pair fills one packed word
-            w[e0 >> 1] = mg[0] | (mg[1] << 16);
-            w[e1 >> 1] = mg[2] | (mg[3] << 16);
+            w[e0 >> 1] = __byte_perm(m[0], m[1], 0x5410);
+            w[e1 >> 1] = __byte_perm(m[2], m[3], 0x5410);
+            if (top <= 65535u) {
+                store4(row, v);
+            } else {
+                const uint4 full = row_full(row, at0 + Sh::row_offset(r, nx, plane), inv, q, qbits, qval, status);
+                w[e0 >> 1] = full.x;
+                w[e1 >> 1] = full.y;
+                neg = full.z;
+            }
+            nm |= ((neg & 3u) << e0) | ((neg >> 2) << e1);
+        }
+    }
+
+    // A row with a code of more than 16 bits or a value that is not finite:
+    // sample by sample (`first`: its index in the field). Returns its two
+    // packed words and its negative mask.
+    static __device__ __noinline__ uint4 row_full(T* row, uint32_t first, T inv, T q, uint32_t* qbits, uint32_t* qval,
+                                                  uint32_t* status) {
+        uint4 out = make_uint4(0, 0, 0, 0);
+        uint32_t bad = 0;
+#pragma unroll 1
+        for (int x = 0; x < 4; ++x) {
+            int32_t m;
+            bool neg;
+            row[x] = quantize_one<T>(row[x], inv, q, m, neg, bad);
+            const uint32_t low = uint32_t(m > 65535 ? 65535 : m) << (16 * (x & 1));
+            if (x < 2) out.x |= low;
+            else out.y |= low;
+            out.z |= uint32_t(neg && m) << x;
+            if (m > 65535) {
+                const uint32_t at = first + x;
+                atomicOr(&qbits[at >> 5], 1u << (at & 31));
+                qval[at] = uint32_t(m);
+            }
         }
         if (bad) atomicOr(status, ST_QUANT_DOMAIN);
+        return out;
     }
 
     // One thread per 16-sample block (thread t: Morton slots 16t .. 16t+15 of
@@ -419,25 +506,25 @@ template <class T> struct QuantBricks {
     __device__ __forceinline__ void block_planes(WzpEncodeSmem& S, uint32_t first, uint32_t count, int tid) const {
         const uint32_t blocks = count >> 4, t = uint32_t(tid);
         uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        uint32_t zm = 0, nm = 0;
+        uint32_t nm = 0;
         if (t < blocks) {
-            if (bz == 16) quantise_block<true>(first, t, w, zm, nm);
-            else quantise_block<false>(first, t, w, zm, nm);
+            if (bz == 16) quantise_block<true>(first, t, w, nm);
+            else quantise_block<false>(first, t, w, nm);
         }
         uint4* dm = reinterpret_cast<uint4*>(S.m + 16 * t);
-
         dm[0] = make_uint4(w[0], w[1], w[2], w[3]);
         dm[1] = make_uint4(w[4], w[5], w[6], w[7]);
+        if ((w[0] | w[1] | w[2] | w[3] | w[4] | w[5] | w[6] | w[7]) != 0) bit_transpose16(w);
         // group statistics: this block's count and compacted signs, merged
         // with the odd neighbour's by the even thread of the pair
-        const uint32_t cnt = __popc(zm), cs = compress16(nm, zm);
+        const uint32_t zm = planes_nonzero(w);
+        const uint32_t cnt = __popc(zm), cs = nm ? compress16(nm, zm, S.pack) : 0u;
         const uint32_t cnt1 = __shfl_xor_sync(0xffffffffu, cnt, 1), cs1 = __shfl_xor_sync(0xffffffffu, cs, 1);
-        if (!(t & 1) && t < kChunk / 16) {
+        if (!(t & 1)) {
             S.gcount[t >> 1] = cnt + cnt1;
             S.gsign[t >> 1] = cs | (cs1 << cnt);
         }
         if (t < blocks) {
-            if ((w[0] | w[1] | w[2] | w[3] | w[4] | w[5] | w[6] | w[7]) != 0) bit_transpose16(w);
             uint16_t* pl = reinterpret_cast<uint16_t*>(S.planes);
             const bool full = blocks == kChunk / 16;
             const uint32_t stride = full ? 2 * kEncPitch : blocks;
@@ -445,70 +532,12 @@ template <class T> struct QuantBricks {
             for (int p = 0; p < 16; ++p) pl[p * stride + t] = uint16_t(p & 1 ? w[p >> 1] >> 16 : w[p >> 1]);
         }
     }
-    __device__ __forceinline__ void load(WzpEncodeSmem& S, uint32_t first, uint32_t count, int tid) const {
-        const uint32_t bsz = 1u << lb, nb = count >> lb, plane = nx * ny;
-        if (tid < int(nb)) {
-            const uint32_t b = (first >> lb) + tid, nbx = nx / 16, nby = ny / 16;
-            const uint32_t bxi = b % nbx, t = b / nbx, byi = t % nby, slab = t / nby;
-            S.bbase[tid] = slab * bz * plane + byi * 16 * nx + bxi * 16;
-        }
-        for (uint32_t e = nb * bsz + tid; e < kChunk; e += kWzpThreads) {
-            S.m[e] = 0;
-            S.sneg[e] = 0;
-        }
-        __syncthreads();
-        uint32_t bad = 0;
-        auto place = [&](uint32_t at, uint32_t slot, int32_t m, bool neg) {
-            S.m[slot] = uint16_t(m > 65535 ? 65535 : m);
-            S.sneg[slot] = neg && m;
-            if (m > 65535) {
-                atomicOr(&qbits[at >> 5], 1u << (at & 31));
-                qval[at] = uint32_t(m);
-            }
-        };
-        if (((reinterpret_cast<uintptr_t>(coeff) & 15u) | (reinterpret_cast<uintptr_t>(rank) & 7u)) == 0) {
-            // four consecutive samples of a brick row per step (16 | nx, so a
-            // row's quarter is 16-byte aligned): one vector load and store of
-            // the coefficients, one 8-byte load of their four ranks
-            for (uint32_t e = 4 * uint32_t(tid); e < nb * bsz; e += 4 * kWzpThreads) {
-                const uint32_t j = e >> lb, i = e & (bsz - 1u);
-                const uint32_t at = S.bbase[j] + (i >> 8) * plane + ((i >> 4) & 15u) * nx + (i & 15u);
-                T v[4];
-                load4(coeff + at, v);
-                const uint2 rk = *reinterpret_cast<const uint2*>(rank + i);
-                const uint32_t base = j << lb;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    int32_t m;
-                    bool neg;
-                    v[k] = quantize_one<T>(v[k], inv, q, m, neg, bad);
-                    const uint32_t r = ((k < 2 ? rk.x : rk.y) >> (16 * (k & 1))) & 0xffffu;
-                    place(at + k, base + r, m, neg);
-                }
-                store4(coeff + at, v);
-            }
-        } else {
-            for (uint32_t e = tid; e < nb * bsz; e += kWzpThreads) {
-                const uint32_t j = e >> lb, i = e & (bsz - 1u);
-                const uint32_t at = S.bbase[j] + (i >> 8) * plane + ((i >> 4) & 15u) * nx + (i & 15u);
-                int32_t m;
-                bool neg;
-                coeff[at] = quantize_one<T>(coeff[at], inv, q, m, neg, bad);
-                place(at, (j << lb) + rank[i], m, neg);
-            }
-        }
-        if (bad) atomicOr(status, ST_QUANT_DOMAIN);
-        __syncthreads();
-        for (uint32_t g = tid; g < kChunk / 32; g += kWzpThreads) {
-            const uint32_t* f = reinterpret_cast<const uint32_t*>(S.sneg + 32 * g);
-            uint32_t bits = 0;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) bits |= (((f[k] & 0x01010101u) * 0x01020408u) >> 24) << (4 * k);
-            S.nsign[g] = bits;
-        }
-    }
 };
 
+// Bound by the ALU pipe (about 60 instructions per sample, seven barriers a
+// chunk; four CTAs per SM overlap them). 512^3 f32: 0.41 ms (2.9 TB/s of read,
+// rewrite and archive); 0.50 ms with per-sample masks, shift-network compress
+// and fourteen barriers a chunk.
 template <class Src> struct WzpEncodeOp {
     static constexpr int kThreads = kWzpThreads, kMinBlocks = 4; // 32 registers: four CTAs per SM
     struct Params {
@@ -537,6 +566,7 @@ __device__ __forceinline__ void WzpEncodeOp<Src>::run(const Params P, uint32_t, 
             }
         S.sel[tid] = sel;
     }
+    if (tid >= 256) S.pack[tid - 256] = uint8_t(pack_entry(uint32_t(tid) - 256u));
     __syncthreads();
     const uint32_t c = S.chunk;
     if (c >= chunks) return;
@@ -614,26 +644,11 @@ __device__ __forceinline__ void WzpEncodeOp<Src>::run(const Params P, uint32_t, 
     __syncthreads();
     }
 
-    // ---- signs: each group's packed sign bits go to its rank offset (at most
-    // two words)
-    uint32_t nnz;
-    {
-        const uint32_t gc = tid < int(kChunk / 32) ? S.gcount[tid] : 0;
-        const uint32_t r = block_excl_scan<kWzpThreads>(gc, S.tmp, nnz);
-        if (tid < int(kChunk / 32)) {
-            const uint32_t packed = S.gsign[tid];
-            if (packed) {
-                const uint32_t sh = r & 31;
-                atomicOr(&S.sgn[r >> 5], packed << sh);
-                if (sh && (packed >> (32 - sh))) atomicOr(&S.sgn[(r >> 5) + 1], packed >> (32 - sh));
-            }
-        }
-    }
-    __syncthreads();
-
-    // ---- zero elimination of the plane bytes: thread t owns bytes 32t..32t+31
+    // ---- zero elimination of the plane bytes (thread t owns bytes
+    // 32t..32t+31, all of one plane in a warp of a full chunk) and the rank
+    // offsets of the 32-groups' signs, from one block scan of both counts
     const uint32_t raw_bytes = 2 * count;
-    uint32_t nzb, c1 = 0, c2 = 0, c3 = 0;
+    uint32_t nnz, nzb, c1 = 0;
     {
         const uint32_t b0 = tid * 32;
         uint32_t w[8];
@@ -642,20 +657,34 @@ __device__ __forceinline__ void WzpEncodeOp<Src>::run(const Params P, uint32_t, 
         const uint4 q0 = q[0], q1 = q[1];
         w[0] = q0.x; w[1] = q0.y; w[2] = q0.z; w[3] = q0.w;
         w[4] = q1.x; w[5] = q1.y; w[6] = q1.z; w[7] = q1.w;
-        uint32_t bits = 0;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) bits |= nonzero_nibble(w[k]) << (4 * k);
+        uint32_t bits = nonzero_mask(w);
         if (b0 + 32 > raw_bytes) bits &= b0 >= raw_bytes ? 0u : ((1u << (raw_bytes - b0)) - 1u);
-        uint32_t o = block_excl_scan<kWzpThreads>(__popc(bits), S.tmp, nzb);
+        const uint32_t gc = tid < int(kChunk / 32) ? S.gcount[tid] : 0u;
+        uint32_t sum;
+        const uint32_t at = block_excl_scan1<kWzpThreads>((uint32_t(__popc(bits)) << 16) | gc, S.tmp[0], sum);
+        nzb = sum >> 16;
+        nnz = sum & 0xffffu;
+        // signs: each group's packed bits at its rank offset (at most two words)
+        if (gc) {
+            const uint32_t r = at & 0xffffu, packed = S.gsign[tid], sh = r & 31;
+            if (packed) {
+                atomicOr(&S.sgn[r >> 5], packed << sh);
+                if (sh && (packed >> (32 - sh))) atomicOr(&S.sgn[(r >> 5) + 1], packed >> (32 - sh));
+            }
+        }
+        // the empty high planes leave here warp by warp
+        if (__any_sync(0xffffffffu, bits)) {
+            uint32_t o = at >> 16;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) o += put_selected(S.planes, o, w[k], (bits >> (4 * k)) & 15u, S.sel);
+            for (int k = 0; k < 8; ++k) o += put_selected(S.planes, o, w[k], (bits >> (4 * k)) & 15u, S.sel);
+        }
         reinterpret_cast<uint32_t*>(S.lv)[tid] = bits; // bitmap bytes 4t..4t+3
     }
     __syncthreads();
     // ---- repetition elimination: 2048 -> 256 -> 32 -> 4 bytes; a byte is
-    // kept iff it differs from the byte before it (before the first: 0)
+    // kept iff it differs from the byte before it (before the first: 0).
+    // Level 1: thread t < 256 owns bitmap bytes 8t..8t+7
     {
-        // level 1: thread t < 256 owns bitmap bytes 8t..8t+7
         uint32_t flags = 0, w0 = 0, w1 = 0;
         if (tid < 256) {
             const uint32_t* lw = reinterpret_cast<const uint32_t*>(S.lv);
@@ -663,63 +692,57 @@ __device__ __forceinline__ void WzpEncodeOp<Src>::run(const Params P, uint32_t, 
             w1 = lw[2 * tid + 1];
             const uint32_t prev = tid ? (lw[2 * tid - 1] >> 24) : 0u;
             flags = changed_nibble(w0, prev) | (changed_nibble(w1, w0 >> 24) << 4);
-        }
-        uint32_t o = nzb + block_excl_scan<kWzpThreads>(__popc(flags), S.tmp, c1);
-        if (tid < 256) {
-            o += put_selected(S.planes, o, w0, flags & 15u, S.sel);
-            put_selected(S.planes, o, w1, flags >> 4, S.sel);
             S.lv[2048 + tid] = uint8_t(flags);
         }
-        __syncthreads();
-        // levels 2 and 3 by warp 0
-        if (warp == 0) {
-            const uint32_t* l1 = reinterpret_cast<const uint32_t*>(S.lv + 2048);
-            const uint32_t v0 = l1[2 * lane], v1 = l1[2 * lane + 1];
-            const uint32_t pv = lane ? (l1[2 * lane - 1] >> 24) : 0u;
-            const uint32_t f2 = changed_nibble(v0, pv) | (changed_nibble(v1, v0 >> 24) << 4);
-            const uint32_t n2 = __popc(f2);
-            const uint32_t inc = warp_incl_scan(n2);
-            c2 = __shfl_sync(0xffffffffu, inc, 31);
-            uint32_t o2 = nzb + c1 + inc - n2;
-            o2 += put_selected(S.planes, o2, v0, f2 & 15u, S.sel);
-            put_selected(S.planes, o2, v1, f2 >> 4, S.sel);
-            S.lv[2048 + 256 + lane] = uint8_t(f2);
-            __syncwarp();
-            const uint32_t* l2 = reinterpret_cast<const uint32_t*>(S.lv + 2048 + 256);
-            uint32_t f3 = 0, u0 = 0, u1 = 0;
-            if (lane < 4) {
-                u0 = l2[2 * lane];
-                u1 = l2[2 * lane + 1];
-                const uint32_t pu = lane ? (l2[2 * lane - 1] >> 24) : 0u;
-                f3 = changed_nibble(u0, pu) | (changed_nibble(u1, u0 >> 24) << 4);
-            }
-            const uint32_t n3 = __popc(f3);
-            const uint32_t inc3 = warp_incl_scan(n3);
-            c3 = __shfl_sync(0xffffffffu, inc3, 31);
-            if (lane < 4) {
-                uint32_t o3 = nzb + c1 + c2 + inc3 - n3;
-                o3 += put_selected(S.planes, o3, u0, f3 & 15u, S.sel);
-                put_selected(S.planes, o3, u1, f3 >> 4, S.sel);
-                S.planes[nzb + c1 + c2 + c3 + lane] = uint8_t(f3);
-            }
-            if (lane == 0) {
-                S.tmp[34] = c2;
-                S.tmp[35] = c3;
-            }
+        uint32_t o = nzb + block_excl_scan1<kWzpThreads>(__popc(flags), S.tmp[1], c1); // its barrier publishes the flags
+        if (flags) {
+            o += put_selected(S.planes, o, w0, flags & 15u, S.sel);
+            put_selected(S.planes, o, w1, flags >> 4, S.sel);
         }
-        __syncthreads();
-        c2 = S.tmp[34];
-        c3 = S.tmp[35];
     }
-    const uint32_t rze = nzb ? nzb + c1 + c2 + c3 + 4 : 0;
-    const bool raw = rze + 2 >= raw_bytes;
-    const uint32_t mbytes = raw ? raw_bytes : rze;
+    // ---- warp 0 alone: levels 2 and 3, the chunk's size and its place, by
+    // decoupled lookback over 32 predecessor states per step (the closest
+    // inclusive prefix ends the walk; every wait is bounded)
     const uint32_t sbytes = (nnz + 7) / 8;
-    const uint64_t chunk_bytes = nnz ? uint64_t(mbytes) + sbytes : 0;
-
-    // ---- decoupled lookback by warp 0: 32 predecessor states per step; the
-    // closest inclusive prefix ends the walk. Every wait is bounded.
     if (warp == 0) {
+        const uint32_t* l1 = reinterpret_cast<const uint32_t*>(S.lv + 2048);
+        const uint32_t v0 = l1[2 * lane], v1 = l1[2 * lane + 1];
+        const uint32_t pv = lane ? (l1[2 * lane - 1] >> 24) : 0u;
+        const uint32_t f2_ = changed_nibble(v0, pv) | (changed_nibble(v1, v0 >> 24) << 4);
+        const uint32_t n2 = __popc(f2_);
+        const uint32_t inc = warp_incl_scan(n2);
+        const uint32_t c2 = __shfl_sync(0xffffffffu, inc, 31);
+        uint32_t o2 = nzb + c1 + inc - n2;
+        o2 += put_selected(S.planes, o2, v0, f2_ & 15u, S.sel);
+        put_selected(S.planes, o2, v1, f2_ >> 4, S.sel);
+        S.lv[2048 + 256 + lane] = uint8_t(f2_);
+        __syncwarp();
+        const uint32_t* l2 = reinterpret_cast<const uint32_t*>(S.lv + 2048 + 256);
+        uint32_t f3 = 0, u0 = 0, u1 = 0;
+        if (lane < 4) {
+            u0 = l2[2 * lane];
+            u1 = l2[2 * lane + 1];
+            const uint32_t pu = lane ? (l2[2 * lane - 1] >> 24) : 0u;
+            f3 = changed_nibble(u0, pu) | (changed_nibble(u1, u0 >> 24) << 4);
+        }
+        const uint32_t n3 = __popc(f3);
+        const uint32_t inc3 = warp_incl_scan(n3);
+        const uint32_t c3 = __shfl_sync(0xffffffffu, inc3, 31);
+        if (lane < 4) {
+            uint32_t o3 = nzb + c1 + c2 + inc3 - n3;
+            o3 += put_selected(S.planes, o3, u0, f3 & 15u, S.sel);
+            put_selected(S.planes, o3, u1, f3 >> 4, S.sel);
+            S.planes[nzb + c1 + c2 + c3 + lane] = uint8_t(f3);
+        }
+        const uint32_t rze = nzb ? nzb + c1 + c2 + c3 + 4 : 0;
+        const bool raw = rze + 2 >= raw_bytes;
+        const uint32_t mbytes = raw ? raw_bytes : rze;
+        const uint64_t chunk_bytes = nnz ? uint64_t(mbytes) + sbytes : 0;
+        if (lane == 0) {
+            S.mbytes = mbytes;
+            S.raw = raw;
+        }
+
         const bool publish = c != A.skip_publish;
         if (lane == 0 && publish)
             atomicExch(reinterpret_cast<unsigned long long*>(&A.state[c]),
@@ -771,7 +794,8 @@ __device__ __forceinline__ void WzpEncodeOp<Src>::run(const Params P, uint32_t, 
     // ---- payload: magnitude bytes (eliminated, or the raw magnitudes), then
     // the sign bytes, each copied with word-wide stores
     uint8_t* dst = A.out + size_t(groups) * 4 + size_t(chunks) * 3 + S.excl;
-    copy_to_global(dst, raw ? reinterpret_cast<const uint8_t*>(S.m) : S.planes, mbytes, tid, kWzpThreads);
+    const uint32_t mbytes = S.mbytes;
+    copy_to_global(dst, S.raw ? reinterpret_cast<const uint8_t*>(S.m) : S.planes, mbytes, tid, kWzpThreads);
     copy_to_global(dst + mbytes, reinterpret_cast<const uint8_t*>(S.sgn), sbytes, tid, kWzpThreads);
 }
 
@@ -846,32 +870,65 @@ struct BrickMap {
     }
 };
 
-// Dequantises block t of the chunk starting at `first` (packed magnitudes w,
-// negative mask nm) into the row-major coefficients as four 16-byte rows.
+// Dequantised samples T(+-m) * q of a block row: magnitudes m in the halves of
+// pa (x = 0, 1) and pb (x = 2, 3), signs in bits 0, 1 of sa and sb (never set
+// for m = 0). Float: a half under the exponent byte of 2^23 is 2^23 + m, so
+// one exact subtraction converts it (two samples at a time).
+__device__ __forceinline__ void dequant_row(uint32_t pa, uint32_t pb, uint32_t sa, uint32_t sb, float q, float (&v)[4]) {
+    const f2 down = f2_pack(-8388608.0f, -8388608.0f), q2 = f2_pack(q, q);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t p = h ? pb : pa, s = h ? sb : sa;
+        const f2 m = f2_pack(__uint_as_float(__byte_perm(p, 0x4b000000u, 0x7410)),
+                             __uint_as_float(__byte_perm(p, 0x4b000000u, 0x7432)));
+        float x, y;
+        f2_unpack(f2_mul(f2_add(m, down), q2), x, y);
+        v[2 * h] = __uint_as_float(__float_as_uint(x) ^ (s << 31));
+        v[2 * h + 1] = __uint_as_float(__float_as_uint(y) ^ ((s << 30) & 0x80000000u));
+    }
+}
+__device__ __forceinline__ void dequant_row(uint32_t pa, uint32_t pb, uint32_t sa, uint32_t sb, double q,
+                                            double (&v)[4]) {
+    const uint32_t mg[4] = {pa & 0xffffu, pa >> 16, pb & 0xffffu, pb >> 16};
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+        const double mag = __dmul_rn(double(mg[x]), q);
+        v[x] = (((x < 2 ? sa : sb) >> (x & 1)) & 1u) ? -mag : mag;
+    }
+}
+
+// Dequantises block t of a chunk (packed magnitudes w, negative mask nm) into
+// the row-major coefficients as four 16-byte rows; `brick` is the row-major
+// base of the block's brick.
 template <class T, bool Tall>
-__device__ __forceinline__ void store_block(const BrickMap& map, T* coeff, uint32_t first, uint32_t t,
+__device__ __forceinline__ void store_block(const BrickMap& map, T* coeff, uint32_t brick, uint32_t t,
                                             const uint32_t (&w)[8], uint32_t nm, T q) {
     using Sh = BlockShape<Tall>;
     const uint32_t plane = map.nx * map.ny;
     uint32_t lx, ly, lz;
     block_origin(t & ((1u << (map.lb - 4)) - 1u), map.lb - 8, lx, ly, lz);
-    const uint32_t b = (first >> map.lb) + ((t << 4) >> map.lb);
-    const uint32_t at0 = map.brick_base(b) + lz * plane + ly * map.nx + lx;
+    const uint32_t at0 = brick + lz * plane + ly * map.nx + lx;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         constexpr int dd = Sh::d;
         const int e0 = Sh::e0(r), e1 = e0 + dd;
-        const uint32_t pa = w[e0 >> 1], pb = w[e1 >> 1];
-        const uint32_t mg[4] = {pa & 0xffffu, pa >> 16, pb & 0xffffu, pb >> 16};
         T v4[4];
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-            const int e = (x < 2 ? e0 : e1) + (x & 1);
-            const T mag = Lift<T>::mul(T(mg[x]), q);
-            v4[x] = ((nm >> e) & 1u) ? -mag : mag;
-        }
+        dequant_row(w[e0 >> 1], w[e1 >> 1], nm >> e0, nm >> e1, q, v4);
         store4(coeff + at0 + Sh::row_offset(r, map.nx, plane), v4);
     }
+}
+
+// One word of an expanded repetition level: four entries whose bits in `mask`
+// say that a new stream byte starts there; the others repeat the byte before
+// (`prev` for the first). `at` is the stream position of the first new byte in
+// the staged words `sw`; `rep` the byte_perm selectors of the 16 masks. Sets
+// bad where a new byte equals the byte before it.
+__device__ __forceinline__ uint32_t repeat_word(const uint32_t* sw, uint32_t at, uint32_t mask, uint32_t prev,
+                                                const uint32_t* rep, bool& bad) {
+    const uint32_t wi = at >> 2;
+    const uint32_t word = __byte_perm(__funnelshift_r(sw[wi], sw[wi + 1], 8 * (at & 3u)), prev, rep[mask]);
+    bad |= changed_nibble(word, prev) != mask;
+    return word;
 }
 
 struct WzpDecodeSmem {
@@ -879,14 +936,17 @@ struct WzpDecodeSmem {
     uint16_t m[kChunk + 16];           // staged magnitude bytes, then the decoded magnitudes
     uint8_t sb[1024 + 32];             // staged sign bytes
     uint32_t xsel[16];                 // byte_perm selectors: spread 4-bit-mask bytes into place
+    uint32_t rep[16];                  // byte_perm selectors: expand repeated bytes
+    uint8_t spread[256];               // expanded nibbles: entry 16 * mask + value
     // full chunks: planes at pitch kEncPitch; a partial chunk: natural, then
     // repacked to pitch kPlanePitch
     uint8_t planes[16 * (kEncPitch > kPlanePitch ? kEncPitch : kPlanePitch) * 4];
-    uint8_t lv[2048 + 256 + 32 + 4];
+    uint8_t lv[256];                   // level 1 of the repetition elimination
     uint32_t gprefix[kChunk / 32];
     uint32_t gmask[kChunk / 32];       // nonzero magnitudes of each 32-group
     uint32_t tmp[40];
-    uint32_t off, mbytes, sbytes, raw, bad;
+    uint32_t tmp1[3][kWzpThreads / 32]; // totals of the block scans of whole-brick chunks
+    uint32_t off, mbytes, sbytes, raw, bad, pos;
 };
 
 struct WzpChunkInfo {
@@ -937,6 +997,9 @@ template <class T> struct WzpDecodeArgs {
     uint32_t* status;
 };
 
+// Bound like the encoder (52 instructions per sample, six barriers). 512^3
+// f32: 0.34 ms; 0.46 ms with a block scan and byte loops per repetition level,
+// shift-network expand and per-sample conversions.
 template <class T> struct WzpDecodeOp {
     static constexpr int kThreads = kWzpThreads, kMinBlocks = 4; // 32 registers: four CTAs per SM
     using Params = WzpDecodeArgs<T>;
@@ -1002,7 +1065,15 @@ __device__ __forceinline__ void WzpDecodeOp<T>::run(const Params A, uint32_t blo
         uint32_t sel = 0, k = 0;
         for (int b = 0; b < 4; ++b) sel |= (((tid >> b) & 1) ? k++ : 4u) << (4 * b);
         S.xsel[tid] = sel;
+        sel = 0, k = 4;
+        for (int b = 0; b < 4; ++b) {
+            if ((tid >> b) & 1) k = k == 4 ? 0 : k + 1;
+            sel |= k << (4 * b);
+        }
+        S.rep[tid] = sel;
     }
+    if (tid >= 256) S.spread[tid - 256] = uint8_t(spread_entry(uint32_t(tid) - 256u));
+    if (A.map.fast && tid < int(kChunk >> A.map.lb)) S.bbase[tid] = A.map.brick_base((first >> A.map.lb) + tid);
     __syncthreads();
     const uint8_t* src = mstage + mis_m; // compressed magnitude bytes (RZE chunks)
     const uint8_t* sgn = S.sb + mis_s;
@@ -1013,91 +1084,57 @@ __device__ __forceinline__ void WzpDecodeOp<T>::run(const Params A, uint32_t blo
         for (int i = tid; i < int(kChunk); i += kWzpThreads)
             S.m[i] = i < int(count) ? uint16_t(gsrc[2 * i] | (gsrc[2 * i + 1] << 8)) : 0;
     } else {
-        // ---- undo repetition elimination from the back of the stream
-        uint32_t pos = mbytes - 4;
-        uint8_t* L3 = S.lv + 2048 + 256 + 32;
-        uint8_t* L2 = S.lv + 2048 + 256;
-        uint8_t* L1 = S.lv + 2048;
-        uint8_t* L0 = S.lv;
-        if (tid < 4) L3[tid] = src[pos + tid];
-        __syncthreads();
-        // level 2 (32 bytes) from L3
+        // ---- undo repetition elimination from the back of the stream:
+        // levels 3 to 1 (4, 32 and 256 bytes) by warp 0
+        const uint32_t* sw = reinterpret_cast<const uint32_t*>(mstage);
         if (warp == 0) {
-            const uint32_t mark = uint32_t(L3[0]) | (uint32_t(L3[1]) << 8) | (uint32_t(L3[2]) << 16) | (uint32_t(L3[3]) << 24);
-            const uint32_t cnt = __popc(mark);
-            const bool under = cnt > pos;
-            const uint32_t base = under ? 0 : pos - cnt;
+            uint32_t pos = mbytes - 4;
+            const uint32_t mark = uint32_t(src[pos]) | (uint32_t(src[pos + 1]) << 8) | (uint32_t(src[pos + 2]) << 16) |
+                                  (uint32_t(src[pos + 3]) << 24);
+            uint32_t cnt = __popc(mark);
+            bool under = cnt > pos;
+            uint32_t base = under ? 0 : pos - cnt;
             const uint32_t rank = __popc(mark & ((2u << lane) - 1u)); // inclusive (lane 31 ok: 2u<<31 == 0)
             const uint32_t r = lane == 31 ? cnt : rank;
-            uint8_t v = 0;
+            uint32_t v = 0; // the lane's byte of level 2
             if (!under && r) v = src[base + r - 1];
             if (!under && ((mark >> lane) & 1u)) {
-                const uint8_t prev = r > 1 ? src[base + r - 2] : 0;
+                const uint32_t prev = r > 1 ? src[base + r - 2] : 0;
                 if (v == prev) bad = true;
             }
-            L2[lane] = v;
-            if (under) bad = true;
-            if (lane == 0) S.tmp[36] = base;
+            bad |= under;
+            // level 1: eight entries per lane
+            pos = base;
+            const uint32_t mine = __popc(v), inc = warp_incl_scan(mine), ex = inc - mine;
+            cnt = __shfl_sync(0xffffffffu, inc, 31);
+            under = cnt > pos;
+            base = under ? 0 : pos - cnt;
+            bad |= under;
+            const uint32_t prev = ex ? src[base + ex - 1] : 0u;
+            const uint32_t a = repeat_word(sw, mis_m + base + ex, v & 15u, prev, S.rep, bad);
+            const uint32_t b = repeat_word(sw, mis_m + base + ex + __popc(v & 15u), v >> 4, a >> 24, S.rep, bad);
+            reinterpret_cast<uint2*>(S.lv)[lane] = make_uint2(a, b);
+            if (lane == 0) S.pos = base;
         }
         __syncthreads();
-        pos = S.tmp[36];
-        // level 1 (256 bytes) from L2
+        uint32_t pos = S.pos;
+        // level 0 (2048 bytes): four entries per thread, which are the bitmap
+        // word of the thread's 32 plane bytes
+        uint32_t bits;
         {
-            uint32_t bit = 0;
-            if (tid < 256) bit = (L2[tid >> 3] >> (tid & 7)) & 1u;
+            const uint32_t mask = (uint32_t(S.lv[tid >> 1]) >> (4 * (tid & 1))) & 15u;
             uint32_t cnt;
-            const uint32_t ex = block_excl_scan<kWzpThreads>(bit, S.tmp, cnt);
+            const uint32_t ex = block_excl_scan1<kWzpThreads>(__popc(mask), S.tmp1[0], cnt);
             const bool under = cnt > pos;
             const uint32_t base = under ? 0 : pos - cnt;
-            if (tid < 256) {
-                const uint32_t r = ex + bit;
-                uint8_t v = 0;
-                if (!under && r) v = src[base + r - 1];
-                if (!under && bit) {
-                    const uint8_t prev = r > 1 ? src[base + r - 2] : 0;
-                    if (v == prev) bad = true;
-                }
-                L1[tid] = v;
-            }
-            if (under) bad = true;
+            bad |= under;
+            bits = repeat_word(sw, mis_m + base + ex, mask, ex ? src[base + ex - 1] : 0u, S.rep, bad);
             pos = base;
         }
-        __syncthreads();
-        // level 0 (2048 bytes) from L1: four entries per thread
-        {
-            uint32_t bits4 = 0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int i = tid * 4 + k;
-                bits4 |= ((L1[i >> 3] >> (i & 7)) & 1u) << k;
-            }
-            uint32_t cnt;
-            const uint32_t ex = block_excl_scan<kWzpThreads>(__popc(bits4), S.tmp, cnt);
-            const bool under = cnt > pos;
-            const uint32_t base = under ? 0 : pos - cnt;
-            uint32_t r = ex;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint32_t bit = (bits4 >> k) & 1u;
-                r += bit;
-                uint8_t v = 0;
-                if (!under && r) v = src[base + r - 1];
-                if (!under && bit) {
-                    const uint8_t prev = r > 1 ? src[base + r - 2] : 0;
-                    if (v == prev) bad = true;
-                }
-                L0[tid * 4 + k] = v;
-            }
-            if (under) bad = true;
-            pos = base;
-        }
-        __syncthreads();
         // nonzero bytes: 32 per thread
         {
-            const uint32_t bits = uint32_t(L0[4 * tid]) | (uint32_t(L0[4 * tid + 1]) << 8) |
-                                  (uint32_t(L0[4 * tid + 2]) << 16) | (uint32_t(L0[4 * tid + 3]) << 24);
             uint32_t cnt;
-            const uint32_t ex = block_excl_scan<kWzpThreads>(__popc(bits), S.tmp, cnt);
+            const uint32_t ex = block_excl_scan1<kWzpThreads>(__popc(bits), S.tmp1[1], cnt);
             if (cnt == 0 || cnt != pos) bad = true;
             const uint32_t b0 = tid * 32;
             // bitmap beyond the chunk's bytes must be empty
@@ -1107,22 +1144,19 @@ __device__ __forceinline__ void WzpDecodeOp<T>::run(const Params A, uint32_t blo
                 if (bits & ~allowed) bad = true;
             }
             // spread the next popc(mask) stream bytes over each word's set
-            // bytes; every one of them must be nonzero and inside the stream
-            uint32_t r = ex;
-            if (r + __popc(bits) > pos) bad = true;
-            const uint32_t* sw = reinterpret_cast<const uint32_t*>(mstage);
-            uint32_t words[8];
+            // bytes; every one of them must be nonzero (all lie inside the
+            // stream when the counts agree). Empty planes pass warp by warp.
+            uint32_t words[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            if (__any_sync(0xffffffffu, bits)) {
+                uint32_t b = mis_m + ex;
 #pragma unroll
-            for (int w = 0; w < 8; ++w) {
-                const uint32_t m4 = (bits >> (4 * w)) & 15u;
-                const uint32_t b = mis_m + r, wi = b >> 2;
-                const uint32_t val = __funnelshift_r(sw[wi], sw[wi + 1], 8 * (b & 3u));
-                const uint32_t word = __byte_perm(val, 0u, S.xsel[m4]);
-                if (nonzero_nibble(word) != m4) bad = true;
-                words[w] = bad ? 0u : word;
-                r += __popc(m4);
+                for (int w = 0; w < 8; ++w) {
+                    const uint32_t m4 = (bits >> (4 * w)) & 15u, wi = b >> 2;
+                    words[w] = __byte_perm(__funnelshift_r(sw[wi], sw[wi + 1], 8 * (b & 3u)), 0u, S.xsel[m4]);
+                    b += __popc(m4);
+                }
+                if (nonzero_mask(words) != bits) bad = true;
             }
-            __syncthreads(); // every thread has read the staged bytes it needs
             // full chunks write the padded layout (plane t / 32 at pitch
             // kEncPitch) straight away; a partial chunk writes the natural one
             const uint32_t pad = blocks == kChunk / 16 ? 4 * (kEncPitch - kChunk / 32) * (uint32_t(tid) >> 5) : 0u;
@@ -1130,16 +1164,17 @@ __device__ __forceinline__ void WzpDecodeOp<T>::run(const Params A, uint32_t blo
             out[0] = make_uint4(words[0], words[1], words[2], words[3]);
             out[1] = make_uint4(words[4], words[5], words[6], words[7]);
         }
-        __syncthreads();
+        const bool full = blocks == kChunk / 16;
         // the verbatim tail (samples past the last whole block) while a
         // partial chunk's planes are still in the natural layout
-        const uint16_t* pl = reinterpret_cast<const uint16_t*>(S.planes);
         uint16_t tail = 0;
         const uint32_t ti = blocks * 16 + tid;
-        if (ti < count) tail = pl[ti];
-        const bool full = blocks == kChunk / 16;
-        if (!full) planes_repack(S.planes, blocks, true, tid);
-        __syncthreads();
+        if (!full || !blockwise) {
+            __syncthreads();
+            if (ti < count) tail = reinterpret_cast<const uint16_t*>(S.planes)[ti];
+            if (!full) planes_repack(S.planes, blocks, true, tid);
+            __syncthreads();
+        }
         if (!blockwise) { // else each thread transposes its own block below
         // ---- inverse bit planes, two groups per warp step: lane l holds plane
         // l % 16 of group g0 + l / 16 (bit 31-e = magnitude e's bit 15-p); one
@@ -1180,29 +1215,28 @@ __device__ __forceinline__ void WzpDecodeOp<T>::run(const Params A, uint32_t blo
         // dequantised block stored as four 16-byte rows
         const uint32_t t = uint32_t(tid);
         uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        uint32_t zm = 0; // bit j: magnitude j is not zero
         if (t < blocks && mbytes != 0) {
             if (S.raw) {
                 const uint4* sm = reinterpret_cast<const uint4*>(S.m + 16 * t);
                 const uint4 a = sm[0], b = sm[1];
                 w[0] = a.x, w[1] = a.y, w[2] = a.z, w[3] = a.w, w[4] = b.x, w[5] = b.y, w[6] = b.z, w[7] = b.w;
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    zm |= (uint32_t((w[i] & 0xffffu) != 0) | (uint32_t((w[i] >> 16) != 0) << 1)) << (2 * i);
             } else {
                 const uint16_t* pl = reinterpret_cast<const uint16_t*>(S.planes);
                 const uint32_t stride = blocks == kChunk / 16 ? 2 * kEncPitch : 2 * kPlanePitch;
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                     w[i] = uint32_t(pl[2 * i * stride + t]) | (uint32_t(pl[(2 * i + 1) * stride + t]) << 16);
-                if ((w[0] | w[1] | w[2] | w[3] | w[4] | w[5] | w[6] | w[7]) != 0) bit_transpose16(w);
+                zm = planes_nonzero(w);
+                if (zm) bit_transpose16(w);
             }
-        }
-        uint32_t zm = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t nzh = __vsetne2(w[i], 0u); // 0xffff per nonzero half
-            zm |= ((nzh & 1u) | ((nzh >> 15) & 2u)) << (2 * i);
         }
         const uint32_t cnt = __popc(zm);
         uint32_t nnz;
-        const uint32_t base = block_excl_scan<kWzpThreads>(cnt, S.tmp, nnz);
+        const uint32_t base = block_excl_scan1<kWzpThreads>(cnt, S.tmp1[2], nnz);
         if (mbytes != 0) {
             if (nnz == 0 || (nnz + 7) / 8 != sbytes) bad = true;
             else if ((nnz & 7) && (sgn[sbytes - 1] >> (nnz & 7))) bad = true;
@@ -1212,10 +1246,11 @@ __device__ __forceinline__ void WzpDecodeOp<T>::run(const Params A, uint32_t blo
             if (cnt && !bad) {
                 const uint32_t by = base >> 3;
                 const uint32_t bits = uint32_t(sgn[by]) | (uint32_t(sgn[by + 1]) << 8) | (uint32_t(sgn[by + 2]) << 16);
-                nm = expand16((bits >> (base & 7u)) & ((1u << cnt) - 1u), zm);
+                nm = expand16(bits >> (base & 7u), zm, S.spread);
             }
-            if (A.map.bz == 16) store_block<T, true>(A.map, A.coeff, first, t, w, nm, q);
-            else store_block<T, false>(A.map, A.coeff, first, t, w, nm, q);
+            const uint32_t brick = S.bbase[(t << 4) >> A.map.lb];
+            if (A.map.bz == 16) store_block<T, true>(A.map, A.coeff, brick, t, w, nm, q);
+            else store_block<T, false>(A.map, A.coeff, brick, t, w, nm, q);
         }
         if (bad) atomicOr(A.status, ST_BAD_STREAM);
         return;
@@ -1230,7 +1265,6 @@ __device__ __forceinline__ void WzpDecodeOp<T>::run(const Params A, uint32_t blo
             S.gmask[g] = nzm;
         }
     }
-    if (A.map.fast && tid < int(kChunk >> A.map.lb)) S.bbase[tid] = A.map.brick_base((first >> A.map.lb) + tid);
     __syncthreads();
     uint32_t nnz = 0;
     {
