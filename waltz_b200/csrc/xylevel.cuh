@@ -77,7 +77,10 @@ template <class Out> struct Prefetching<Out, decltype(void(Out::kPrefetch))> {
 };
 
 template <class T, bool Inverse, class Src, class Out> struct XYMarchOp {
-    static constexpr int kThreads = 256, kMinBlocks = 0; // no occupancy floor: about 80 registers, three CTAs per SM
+    // float: the compiler picks about 80 registers (three CTAs per SM; 115 with
+    // the repair emitter, faster than 80 with spills); double: capped at 128, so
+    // that two CTAs share an SM (96 x 256 x 384 forward: 0.100 -> 0.081 ms)
+    static constexpr int kThreads = 256, kMinBlocks = sizeof(T) == 4 ? 0 : 2;
     struct Params {
         Src src;
         Dims a;   // level dims (x, y lifted; z planes)
