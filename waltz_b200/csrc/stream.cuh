@@ -118,8 +118,10 @@ __device__ __forceinline__ void FwdStreamOp<T, UX, UY, Q, Z, NT>::run(const Para
     const int fx_lo = ox < 4 ? int(4 - ox) : 0, fx_hi = min(S::FX, int(a.x - ox) + 4);
     const int fy_lo = oy < 4 ? int(4 - oy) : 0, fy_hi = min(S::FY, int(a.y - oy) + 4);
 
-    // per-thread output columns: x/y parts of the split addresses
-    size_t hi_off[S::CPT], lo_off[S::CPT];
+    // per-thread output columns: x/y parts of the split addresses, 32 bits (a
+    // field has fewer than 2^32 samples): with 64 the 256-thread float kernel
+    // spilled at its 64 registers (512^3 finest level 0.425 -> 0.367 ms)
+    uint32_t hi_off[S::CPT], lo_off[S::CPT];
     bool even_xy[S::CPT];
     ZPipe<T> pipe[S::CPT];
 #pragma unroll
@@ -127,13 +129,13 @@ __device__ __forceinline__ void FwdStreamOp<T, UX, UY, Q, Z, NT>::run(const Para
         const int k = tid + c * NT;
         const uint32_t x = ox + k % UX, y = oy + k / UX;
         const uint32_t cx = split_of(x, a.x), cy = split_of(y, a.y);
-        hi_off[c] = size_t(cy) * out.sy + cx;
-        lo_off[c] = size_t(cy) * out.lo.x + cx;
+        hi_off[c] = cy * uint32_t(out.sy) + cx;
+        lo_off[c] = cy * out.lo.x + cx;
         even_xy[c] = out.low && !(x & 1) && !(y & 1);
         pipe[c] = ZPipe<T>{T(0), T(0), T(0), T(0), T(0)};
     }
     const uint32_t zhalf = half_len(a.z);
-    const size_t lo_plane = size_t(out.lo.x) * out.lo.y;
+    const uint32_t lo_plane = out.lo.x * out.lo.y, plane = uint32_t(out.sz);
     Bits seen = 0;
 
     auto issue = [&](int64_t zb) { // one thread: arm the barrier and copy Q planes
@@ -263,11 +265,11 @@ __device__ __forceinline__ void FwdStreamOp<T, UX, UY, Q, Z, NT>::run(const Para
                 const T* s = Mid + y * S::YP + x;
 #pragma unroll
                 for (int q = 0; q < Q; ++q) {
-                    const int64_t zo = zb + q;
-                    if (zo >= int64_t(z1)) break;
+                    const int zo = int(zb) + q;
+                    if (zo >= int(z1)) break;
                     const T v = s[q * UY * S::YP];
-                    if (even_xy[c]) out.low[size_t(zo) * lo_plane + lo_off[c]] = v;
-                    else out.dst[size_t(zo) * out.sz + hi_off[c]] = v;
+                    if (even_xy[c]) out.low[uint32_t(zo) * lo_plane + lo_off[c]] = v;
+                    else out.dst[uint32_t(zo) * plane + hi_off[c]] = v;
                 }
             }
         } else {
@@ -287,13 +289,13 @@ __device__ __forceinline__ void FwdStreamOp<T, UX, UY, Q, Z, NT>::run(const Para
                     const T e2 = L::fma(K97<T>::b, L::add(p.o1, o1), p.e);
                     const T o3 = L::fma(K97<T>::g, L::add(p.e2, e2), p.o1);
                     const T e4 = L::fma(K97<T>::d, L::add(p.o3, o3), p.e2);
-                    const int64_t zo = zb + q - 4; // even output plane of this pair
-                    if (inside && zo >= int64_t(z0) && zo < int64_t(z1)) {
-                        const size_t cz = size_t(zo) >> 1;
+                    const int zo = int(zb) + q - 4; // even output plane of this pair
+                    if (inside && zo >= int(z0) && zo < int(z1)) {
+                        const uint32_t cz = uint32_t(zo) >> 1;
                         const T ev = L::mul(e4, K97<T>::k);
                         if (even_xy[c]) out.low[cz * lo_plane + lo_off[c]] = ev;
-                        else out.dst[cz * out.sz + hi_off[c]] = ev;
-                        if (zo + 1 < int64_t(z1)) out.dst[(zhalf + cz) * out.sz + hi_off[c]] = L::mul(o3, -K97<T>::ik);
+                        else out.dst[cz * plane + hi_off[c]] = ev;
+                        if (zo + 1 < int(z1)) out.dst[(zhalf + cz) * plane + hi_off[c]] = L::mul(o3, -K97<T>::ik);
                     }
                     p.o3 = o3;
                     p.e2 = e2;
