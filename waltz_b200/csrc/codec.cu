@@ -1138,7 +1138,7 @@ template <class T> struct CompressJob {
         T *C, *lowA, *lowB, *inter, *bank2, *perr;
         uint16_t* mag;
         uint32_t *sign, *qbits, *qval, *pbits, *status, *ticket, *counts_p, *counts_q;
-        uint64_t *state, *sizes, *wzp_total, *layout; // layout[8] = status copy
+        uint64_t *state, *sizes, *layout; // layout[8] = status copy
         uint32_t* wpw_groups;  // compact repairs: per group bytes, then offsets
         uint64_t* wpw_state;
         uint8_t* wpw_tail;     // the compact section and the moved q-outlier sections
@@ -1193,7 +1193,6 @@ template <class T> struct CompressJob {
         p.counts_p = c.take<uint32_t>(cblocks);
         p.counts_q = c.take<uint32_t>(cblocks);
         p.sizes = c.take<uint64_t>(chunks);
-        p.wzp_total = c.take<uint64_t>(1);
         p.layout = c.take<uint64_t>(9);
         p.wpw_groups = nullptr;
         p.wpw_state = nullptr;
@@ -1258,10 +1257,6 @@ template <class T> struct CompressJob {
             } else {
                 launch_wzp_encode(wa, MagArrays{P.mag, P.sign}, chunks, sink);
             }
-            sink.phase(PH_DIRECTORY);
-            const uint32_t groups = wzp_groups(uint32_t(n));
-            sink.run<WzpDirectoryOp>(WzpDirectoryOp::Params{out + 32, uint32_t(n), P.state, P.sizes, P.wzp_total},
-                                     (groups + 255) / 256);
         }
         sink.mark("wzp_encode");
         // 4. inverse transform + repairs; fast-accept threshold of the repair
@@ -1279,7 +1274,7 @@ template <class T> struct CompressJob {
         sink.run<CompactCountOp>(CompactCountOp::Params{P.pbits, P.qbits, words, P.counts_p, P.counts_q,
                                                         uint32_t(cblocks)},
                                  both);
-        sink.run<ScanLayoutOp>(ScanLayoutOp::Params{P.counts_p, P.counts_q, uint32_t(cblocks), P.wzp_total, P.status,
+        sink.run<ScanLayoutOp>(ScanLayoutOp::Params{P.counts_p, P.counts_q, uint32_t(cblocks), uint32_t(n), P.state, P.sizes, P.status,
                                                     out, capacity, uint32_t(sizeof(T)),
                                                     uint8_t(g.flags(sizeof(T)) | split_flags(opt.zsplit)),
                                                     uint8_t(g.lxy), uint8_t(g.lz), split_band(opt.zsplit, g.bz), quantum, layout},
@@ -1340,6 +1335,7 @@ static size_t compress(const T* d_in, uint32_t nx, uint32_t ny, uint32_t nz, dou
     char* scratch = t_arena.reserve(job.scratch_bytes());
     const uint16_t* rank = t_fwd_tables.get(nx, ny, nz, job.g.bz, false, stream);
     Sink sink{stream};
+    sink.chained = true;
     job.enqueue(scratch, rank, sink);
     uint64_t* h = pinned();
     check(cudaMemcpyAsync(h, job.result(scratch), 9 * 8, cudaMemcpyDeviceToHost, stream), "readback");
@@ -1424,56 +1420,8 @@ static Layout validate_header(const Header& h, const Geometry& g, size_t bytes, 
     return L;
 }
 
-// Directory check: group spans must tile the payload exactly. The fast path
-// verifies canonical (increasing) order on the device; anything else is
-// checked on the host like cpu/src/wzp_cpu.cpp:720-761.
-struct DirectoryCheckOp {
-    static constexpr int kThreads = 1024, kMinBlocks = 0; // no occupancy floor: the compiler picks the register budget
-    struct Params {
-        JobRef job;
-        uint32_t n;
-        uint32_t* status;
-    };
-    static __device__ __forceinline__ void run(const Params P, uint32_t, uint32_t);
-};
-
-__device__ __forceinline__ void DirectoryCheckOp::run(const Params P, uint32_t, uint32_t) {
-    const uint32_t n = P.n;
-    uint32_t* const status = P.status;
-    const JobRef& job = P.job;
-    __shared__ uint32_t tmp[40];
-    const DecodeJob J = job.get();
-    const uint8_t* in = J.base + 32;
-    const uint64_t payload = J.wzp - wzp_header(n);
-    const uint32_t chunks = wzp_chunks(n), groups = wzp_groups(n);
-    const uint8_t* meta = in + size_t(groups) * 4;
-    uint64_t carry = 0;
-    uint32_t st = 0;
-    for (uint32_t base = 0; base < groups; base += kThreads) {
-        const uint32_t g = base + threadIdx.x;
-        uint32_t len = 0, off = 0;
-        if (g < groups) {
-            // the group's 16 metadata words are independent loads: all in flight at once
-#pragma unroll
-            for (uint32_t k = 0; k < kGroup; ++k) {
-                const uint32_t c = g * kGroup + k;
-                if (c >= chunks) break;
-                const WzpChunkInfo ci = wzp_meta(load_u24(meta + size_t(c) * 3), min(kChunk, n - c * kChunk));
-                if (!ci.ok) st |= ST_BAD_STREAM;
-                len += ci.mbytes + ci.sbytes;
-            }
-            off = load_u32(in + size_t(g) * 4);
-            if (off > payload || len > payload - off || (!len && off)) st |= ST_BAD_STREAM;
-        }
-        uint32_t sum;
-        const uint32_t ex = block_excl_scan<kThreads>(len, tmp, sum);
-        if (g < groups && len && uint64_t(off) != carry + ex) st |= ST_DIRECTORY;
-        carry += sum;
-    }
-    if (threadIdx.x == 0 && carry != payload) st |= ST_DIRECTORY;
-    if (st) atomicOr(status, st);
-}
-
+// Exact host check of a WZP directory that is not in the canonical order
+// (directory_check), like cpu/src/wzp_cpu.cpp:720-761.
 static void host_directory_check(const uint8_t* in, uint32_t n, uint64_t payload) {
     const uint32_t chunks = wzp_chunks(n), groups = wzp_groups(n);
     std::vector<std::pair<uint32_t, uint32_t>> spans;
@@ -1521,8 +1469,6 @@ static void decode_launch(const JobRef& job, int zsplit, const Geometry& g, cons
                           T* bank2, const Final& fin, const Patch& patch, uint32_t* status, Sink& sink) {
     const uint32_t n = uint32_t(g.n);
     if (!sink.rec) stage_clock().begin(sink.stream);
-    sink.phase(PH_DCHECK);
-    sink.run<DirectoryCheckOp>(DirectoryCheckOp::Params{job, n, status}, 1);
     {
         sink.phase(PH_DECODE);
         BrickMap map{g.nx, g.ny, g.nz, g.bz, irank, frank, false, 0};
@@ -1532,7 +1478,8 @@ static void decode_launch(const JobRef& job, int zsplit, const Geometry& g, cons
             map.fast = true;
             while ((1u << map.lb) < bsz) ++map.lb;
         }
-        sink.run<WzpDecodeOp<T>>(WzpDecodeArgs<T>{job, n, map, C, status}, wzp_chunks(n), sizeof(WzpDecodeSmem));
+        // block 0 checks the directory meanwhile
+        sink.run<WzpDecodeOp<T>>(WzpDecodeArgs<T>{job, n, map, C, status}, wzp_chunks(n) + 1, sizeof(WzpDecodeSmem));
     }
     sink.mark("wzp_decode");
     const uint32_t fixed = uint32_t(std::min<uint64_t>((g.n + 255) / 256, 32));
@@ -1637,6 +1584,7 @@ static void decompress(const uint8_t* d_in, size_t bytes, uint32_t nx, uint32_t 
     check(cudaMemsetAsync(P.status, 0, 4, stream), "memset");
     FinalOut<T> fin{d_out, nx, size_t(nx) * ny, P.status};
     Sink sink{stream};
+    sink.chained = true;
     decode_launch<T>(JobRef{nullptr, decode_job(d_in, h, L)}, h.split, g, irank, frank, P.C, P.bank1,
                      P.bank2, fin, RowPatch<T>{d_out}, P.status, sink);
     check(cudaMemcpyAsync(pin + 8, P.status, 4, cudaMemcpyDeviceToHost, stream), "readback");

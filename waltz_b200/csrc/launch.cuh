@@ -30,15 +30,27 @@ template <class K> static void opt_in_smem(K kernel, size_t bytes, int& device, 
     }
 }
 
-template <class Op> static void launch_op(const typename Op::Params& p, uint32_t blocks, size_t smem, cudaStream_t s) {
+// `chained`: launched as the programmatic successor of the stream's last kernel
+// (stage_enter orders them).
+template <class Op>
+static void launch_op(const typename Op::Params& p, uint32_t blocks, size_t smem, cudaStream_t s, bool chained) {
     if (!blocks) return;
     static thread_local int device = -1;
     static thread_local size_t granted = 0;
     constexpr auto kernel = op_kernel_for<Op>();
     opt_in_smem(kernel, smem, device, granted);
-    kernel<<<blocks, Op::kThreads, smem, s>>>(p);
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(Op::kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    check(cudaLaunchKernelEx(&cfg, kernel, p), "kernel launch");
     note_launch();
-    check(cudaGetLastError(), "kernel launch");
 }
 
 template <class Op>
@@ -151,8 +163,8 @@ struct DirectRec final : OpRecord {
 
 // Pipeline phases, in order; a field's stages keep their order inside one.
 enum Phase : int {
-    PH_INIT = 0, PH_FORWARD, PH_QUANT, PH_ENCODE, PH_DIRECTORY, PH_INVERSE, PH_SIDE,
-    PH_DCHECK, PH_DECODE, PH_QPATCH, PH_DINVERSE, PH_RPATCH,
+    PH_INIT = 0, PH_FORWARD, PH_QUANT, PH_ENCODE, PH_INVERSE, PH_SIDE,
+    PH_DECODE, PH_QPATCH, PH_DINVERSE, PH_RPATCH,
 };
 
 struct Recorder {
@@ -174,9 +186,10 @@ struct Sink {
     cudaStream_t stream = nullptr;
     Recorder* rec = nullptr;
     bool many = false; // many fields share the GPU: prefer fewer, larger blocks of work per field
+    bool chained = false; // one field's stages, not captured: each launched ahead of its predecessor's end
     template <class Op> void run(const typename Op::Params& p, uint32_t blocks, size_t smem = 0) {
         if (rec) rec->add(std::make_unique<OpRec<Op>>(p, blocks, smem));
-        else launch_op<Op>(p, blocks, smem, stream);
+        else launch_op<Op>(p, blocks, smem, stream, chained);
     }
     void zero(void* ptr, size_t bytes) {
         if (!bytes) return;

@@ -381,13 +381,19 @@ template <class T> struct CompactWriteOp {
 // Exclusive scan of both lists' block counts in place, then the archive
 // layout from the totals. layout[]: 0 pi, 1 pv, 2 qi, 3 qv, 4 end, 5 np,
 // 6 nq, 7 overflow flag, 8 the pipeline's status word. Also writes the
-// 32-byte header and zeroes every padding byte between sections.
+// 32-byte header and the WZP group directory, and zeroes every padding byte
+// between sections.
+__device__ __forceinline__ void wzp_write_directory(uint8_t* out, uint32_t n, const uint64_t* state,
+                                                    const uint64_t* sizes, uint32_t t, uint32_t step);
+__device__ __forceinline__ uint64_t wzp_stream_bytes(uint32_t n, const uint64_t* state);
+
 struct ScanLayoutOp {
-    static constexpr int kThreads = kCompactThreads, kMinBlocks = 0; // no occupancy floor: the compiler picks the register budget
+    static constexpr int kThreads = 1024, kMinBlocks = 0; // no occupancy floor: the compiler picks the register budget
     struct Params {
         uint32_t *counts_p, *counts_q;
         uint32_t count;
-        const uint64_t* wzp_total;
+        uint32_t n;
+        const uint64_t *state, *sizes; // the encoder's chunk states and sizes
         const uint32_t* status;
         uint8_t* archive;
         size_t capacity;
@@ -403,7 +409,6 @@ __device__ __forceinline__ void ScanLayoutOp::run(const Params P, uint32_t, uint
     uint32_t* const counts_p = P.counts_p;
     uint32_t* const counts_q = P.counts_q;
     const uint32_t count = P.count, width = P.width;
-    const uint64_t* wzp_total = P.wzp_total;
     const uint32_t* status = P.status;
     uint8_t* const archive = P.archive;
     const size_t capacity = P.capacity;
@@ -414,15 +419,15 @@ __device__ __forceinline__ void ScanLayoutOp::run(const Params P, uint32_t, uint
     uint32_t totals[2];
     // each thread takes a run of consecutive block counts: its run's sum, one
     // block scan for the runs' offsets, then the run rewritten as exclusive
-    // prefixes (two block scans in all instead of one per kCompactThreads)
-    const uint32_t per = (count + kCompactThreads - 1) / kCompactThreads;
+    // prefixes (two block scans in all instead of one per kThreads)
+    const uint32_t per = (count + kThreads - 1) / kThreads;
     const uint32_t b0 = min(count, threadIdx.x * per), b1 = min(count, b0 + per);
     for (int list = 0; list < 2; ++list) {
         uint32_t* counts = list ? counts_q : counts_p;
         uint32_t run = 0;
         for (uint32_t i = b0; i < b1; ++i) run += counts[i];
         uint32_t sum;
-        uint32_t at = block_excl_scan<kCompactThreads>(run, tmp, sum);
+        uint32_t at = block_excl_scan<kThreads>(run, tmp, sum);
         for (uint32_t i = b0; i < b1; ++i) {
             const uint32_t v = counts[i];
             counts[i] = at;
@@ -430,8 +435,9 @@ __device__ __forceinline__ void ScanLayoutOp::run(const Params P, uint32_t, uint
         }
         totals[list] = sum;
     }
+    wzp_write_directory(archive + 32, P.n, P.state, P.sizes, threadIdx.x, kThreads);
     if (threadIdx.x != 0) return;
-    const uint64_t wb = *wzp_total; // includes the WZP header
+    const uint64_t wb = wzp_stream_bytes(P.n, P.state); // includes the WZP header
     const uint32_t np = totals[0], nq = totals[1];
     const uint64_t pi = 32 + pad8(wb);
     const uint64_t pv = pi + pad8(uint64_t(np) * 4);

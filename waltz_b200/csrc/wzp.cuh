@@ -799,7 +799,25 @@ __device__ __forceinline__ void WzpEncodeOp<Src>::run(const Params P, uint32_t, 
     copy_to_global(dst + mbytes, reinterpret_cast<const uint8_t*>(S.sgn), sbytes, tid, kWzpThreads);
 }
 
-// Group directory: payload offset of the first byte of every nonempty group.
+// Group directory: payload offset of the first byte of every nonempty group,
+// for groups t, t + step, ...
+__device__ __forceinline__ void wzp_write_directory(uint8_t* out, uint32_t n, const uint64_t* state,
+                                                    const uint64_t* sizes, uint32_t t, uint32_t step) {
+    const uint32_t chunks = wzp_chunks(n), groups = wzp_groups(n);
+    for (uint32_t g = t; g < groups; g += step) {
+        const uint32_t f = g * kGroup, l = min(f + kGroup, chunks) - 1;
+        const uint64_t start = (state[f] & kValueMask) - sizes[f];
+        const uint64_t end = state[l] & kValueMask;
+        store_u32(out + size_t(g) * 4, end > start ? uint32_t(start) : 0u);
+    }
+}
+// Bytes of the whole stream (its header included) once every chunk is done.
+__device__ __forceinline__ uint64_t wzp_stream_bytes(uint32_t n, const uint64_t* state) {
+    return wzp_header(n) + (state[wzp_chunks(n) - 1] & kValueMask);
+}
+
+// The directory of a standalone encode (the compressor writes it with the
+// archive's layout).
 struct WzpDirectoryOp {
     static constexpr int kThreads = 256, kMinBlocks = 0; // no occupancy floor: the compiler picks the register budget
     struct Params {
@@ -808,23 +826,11 @@ struct WzpDirectoryOp {
         const uint64_t *state, *sizes;
         uint64_t* total;
     };
-    static __device__ __forceinline__ void run(const Params P, uint32_t block, uint32_t);
+    static __device__ __forceinline__ void run(const Params P, uint32_t block, uint32_t blocks) {
+        wzp_write_directory(P.out, P.n, P.state, P.sizes, block * kThreads + threadIdx.x, blocks * kThreads);
+        if (block == 0 && threadIdx.x == 0) *P.total = wzp_stream_bytes(P.n, P.state);
+    }
 };
-
-__device__ __forceinline__ void WzpDirectoryOp::run(const Params P, uint32_t block, uint32_t) {
-    uint8_t* const out = P.out;
-    const uint32_t n = P.n;
-    const uint64_t *state = P.state, *sizes = P.sizes;
-    uint64_t* const total = P.total;
-    const uint32_t chunks = wzp_chunks(n), groups = wzp_groups(n);
-    const uint32_t g = block * kThreads + threadIdx.x;
-    if (g >= groups) return;
-    const uint32_t f = g * kGroup, l = min(f + kGroup, chunks) - 1;
-    const uint64_t start = (state[f] & kValueMask) - sizes[f];
-    const uint64_t end = state[l] & kValueMask;
-    store_u32(out + size_t(g) * 4, end > start ? uint32_t(start) : 0u);
-    if (g == groups - 1) *total = size_t(groups) * 4 + size_t(chunks) * 3 + end;
-}
 
 // ------------------------------------------------------------------ decode
 
@@ -968,6 +974,42 @@ __device__ __forceinline__ WzpChunkInfo wzp_meta(uint32_t meta, uint32_t count) 
     return r;
 }
 
+// Directory check by one block of NT threads: group spans must tile the payload
+// exactly. This verifies the canonical (increasing) order; ST_DIRECTORY sends
+// anything else to the exact host check.
+template <int NT>
+__device__ __forceinline__ void directory_check(const DecodeJob& J, uint32_t n, uint32_t* status, uint32_t* tmp) {
+    const uint8_t* in = J.base + 32;
+    const uint64_t payload = J.wzp - wzp_header(n);
+    const uint32_t chunks = wzp_chunks(n), groups = wzp_groups(n);
+    const uint8_t* meta = in + size_t(groups) * 4;
+    uint64_t carry = 0;
+    uint32_t st = 0;
+    for (uint32_t base = 0; base < groups; base += NT) {
+        const uint32_t g = base + threadIdx.x;
+        uint32_t len = 0, off = 0;
+        if (g < groups) {
+            // the group's 16 metadata words are independent loads: all in flight at once
+#pragma unroll
+            for (uint32_t k = 0; k < kGroup; ++k) {
+                const uint32_t c = g * kGroup + k;
+                if (c >= chunks) break;
+                const WzpChunkInfo ci = wzp_meta(load_u24(meta + size_t(c) * 3), min(kChunk, n - c * kChunk));
+                if (!ci.ok) st |= ST_BAD_STREAM;
+                len += ci.mbytes + ci.sbytes;
+            }
+            off = load_u32(in + size_t(g) * 4);
+            if (off > payload || len > payload - off || (!len && off)) st |= ST_BAD_STREAM;
+        }
+        uint32_t sum;
+        const uint32_t ex = block_excl_scan<NT>(len, tmp, sum);
+        if (g < groups && len && uint64_t(off) != carry + ex) st |= ST_DIRECTORY;
+        carry += sum;
+    }
+    if (threadIdx.x == 0 && carry != payload) st |= ST_DIRECTORY;
+    if (st) atomicOr(status, st);
+}
+
 // Copies src[0, len) to dst[mis, mis + len), mis = src mod 16 (dst 16-byte
 // aligned): 16-byte loads for granules wholly inside the range, bytes at its
 // ends. Returns mis.
@@ -1013,7 +1055,13 @@ __device__ __forceinline__ void WzpDecodeOp<T>::run(const Params A, uint32_t blo
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int NW = kWzpThreads / 32;
     const uint32_t chunks = wzp_chunks(A.n), groups = wzp_groups(A.n);
-    const uint32_t c = block;
+    // block 0 checks the directory beside the chunks' blocks (as a launch of
+    // its own it took 4.7 us of every decode)
+    if (block == 0) {
+        directory_check<kWzpThreads>(A.job.get(), A.n, A.status, S.tmp);
+        return;
+    }
+    const uint32_t c = block - 1;
     const uint32_t first = c * kChunk, count = min(kChunk, A.n - first);
     const size_t header = size_t(groups) * 4 + size_t(chunks) * 3;
     const DecodeJob J = A.job.get();
