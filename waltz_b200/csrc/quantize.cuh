@@ -106,28 +106,43 @@ __device__ __forceinline__ void QuantizeOp<T>::run(const Params A, uint32_t bloc
     const uint16_t* rank = A.rank + slot * 256 * B.bz;
     const T* corner = A.coeff + (uint64_t(bzi) * B.bz) * plane + uint64_t(byi) * 16 * B.nx + bxi * 16;
     uint32_t bad = 0;
-    for (uint32_t i = threadIdx.x; i < size; i += kQuantThreads) {
-        uint32_t lx, ly, lz;
-        if (full) {
-            lx = i & 15u;
-            ly = (i >> 4) & 15u;
-            lz = i >> 8;
-        } else {
-            lx = i % ex;
-            ly = (i / ex) % ey;
-            lz = i / (ex * ey);
+    // six samples per thread and round, loaded before the first is used
+    constexpr int U = 6;
+    for (uint32_t i0 = threadIdx.x; i0 < size; i0 += U * kQuantThreads) {
+        T* cp[U];
+        T v[U];
+        uint32_t rk[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t i = i0 + u * kQuantThreads;
+            if (i >= size) break;
+            uint32_t lx, ly, lz;
+            if (full) {
+                lx = i & 15u;
+                ly = (i >> 4) & 15u;
+                lz = i >> 8;
+            } else {
+                lx = i % ex;
+                ly = (i / ex) % ey;
+                lz = i / (ex * ey);
+            }
+            cp[u] = const_cast<T*>(corner) + lz * plane + uint64_t(ly) * B.nx + lx;
+            v[u] = *cp[u];
+            rk[u] = rank[i];
         }
-        T* cp = const_cast<T*>(corner) + lz * plane + uint64_t(ly) * B.nx + lx;
-        int32_t m;
-        bool neg;
-        *cp = quantize_one<T>(*cp, A.inv, A.q, m, neg, bad);
-        const uint32_t rk = rank[i];
-        smag[rk] = uint16_t(m > 65535 ? 65535 : m);
-        ssign[rk] = neg && m;
-        if (m > 65535) {
-            const uint64_t at = uint64_t(cp - A.coeff);
-            atomicOr(&A.qbits[at >> 5], 1u << (at & 31));
-            A.qval[at] = uint32_t(m);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (i0 + u * kQuantThreads >= size) break;
+            int32_t m;
+            bool neg;
+            *cp[u] = quantize_one<T>(v[u], A.inv, A.q, m, neg, bad);
+            smag[rk[u]] = uint16_t(m > 65535 ? 65535 : m);
+            ssign[rk[u]] = neg && m;
+            if (m > 65535) {
+                const uint64_t at = uint64_t(cp[u] - A.coeff);
+                atomicOr(&A.qbits[at >> 5], 1u << (at & 31));
+                A.qval[at] = uint32_t(m);
+            }
         }
     }
     if (bad) atomicOr(A.status, ST_QUANT_DOMAIN);
@@ -147,15 +162,13 @@ __device__ __forceinline__ void QuantizeOp<T>::run(const Params A, uint32_t bloc
         return;
     }
     for (uint32_t i = threadIdx.x; i < size; i += kQuantThreads) A.mag[base + i] = smag[i];
-    // sign words overlapping [base, base+size)
+    // sign words overlapping [base, base+size), one warp vote each
     const uint64_t w0 = base >> 5, w1 = (base + size + 31) >> 5;
-    for (uint64_t w = w0 + threadIdx.x; w < w1; w += kQuantThreads) {
-        uint32_t bits = 0;
-        for (int k = 0; k < 32; ++k) {
-            const uint64_t p = w * 32 + k;
-            if (p >= base && p < base + size && ssign[p - base]) bits |= 1u << k;
-        }
-        if (bits) atomicOr(&A.sign[w], bits);
+    const int lane = threadIdx.x & 31;
+    for (uint64_t w = w0 + threadIdx.x / 32; w < w1; w += kQuantThreads / 32) {
+        const uint64_t p = w * 32 + lane;
+        const uint32_t bits = __ballot_sync(0xffffffffu, p >= base && p < base + size && ssign[p - base]);
+        if (lane == 0 && bits) atomicOr(&A.sign[w], bits);
     }
 }
 

@@ -59,55 +59,9 @@ constexpr uint32_t kEncBytes = 2 * kChunk + 2048 + 256 + 32 + 4 + 28;
 // (8 words of one plane) stay 16-byte aligned and contiguous at natural word
 // 8t plus 4 * (t / 32), so the zero elimination reads them, and the decoder's
 // byte spreading writes them, in place. A partial chunk (a field's last)
-// keeps the natural layout; the decoder repacks it to plane p at u32 word
-// p * kPlanePitch + group by a conflict-free pass (consecutive threads on
-// consecutive natural words).
-constexpr uint32_t kPlanePitch = kChunk / 32 + 1; // u32 words per padded plane, partial chunks
-constexpr uint32_t kEncPitch = kChunk / 32 + 4;   // u32 words per padded plane, full chunks
+// keeps the natural layout.
+constexpr uint32_t kEncPitch = kChunk / 32 + 4; // u32 words per padded plane, full chunks
 static_assert(16 * kEncPitch * 4 <= kEncBytes, "padded encoder planes fit the plane buffer");
-
-// natural -> padded (dir = true) or padded -> natural, in place in `buf`
-// (room for 16 * kPlanePitch words); the caller syncs before and after.
-__device__ __forceinline__ void planes_repack(uint8_t* buf, uint32_t blocks, bool to_padded, int tid) {
-    constexpr int PER = (16 * kChunk / 16 / 2 + kWzpThreads - 1) / kWzpThreads; // u32 words per thread
-    uint32_t* w = reinterpret_cast<uint32_t*>(buf);
-    if (blocks == 0) return; // no whole block: no planes (uniform across the block)
-    if ((blocks & 1u) == 0) {
-        const uint32_t per_plane = blocks / 2, words = 16 * per_plane;
-        uint32_t v[PER];
-#pragma unroll
-        for (int k = 0; k < PER; ++k) {
-            const uint32_t q = tid + k * kWzpThreads;
-            const uint32_t p = q / per_plane, g = q - p * per_plane;
-            if (q < words) v[k] = to_padded ? w[q] : w[p * kPlanePitch + g];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < PER; ++k) {
-            const uint32_t q = tid + k * kWzpThreads;
-            const uint32_t p = q / per_plane, g = q - p * per_plane;
-            if (q < words) (to_padded ? w[p * kPlanePitch + g] : w[q]) = v[k];
-        }
-    } else {
-        // an odd number of 16-sample blocks (a field's last chunk): u16 steps
-        uint16_t* h = reinterpret_cast<uint16_t*>(buf);
-        const uint32_t halves = 16 * blocks;
-        uint16_t v[2 * PER];
-#pragma unroll
-        for (int k = 0; k < 2 * PER; ++k) {
-            const uint32_t q = tid + k * kWzpThreads;
-            const uint32_t p = q / blocks, b = q - p * blocks;
-            if (q < halves) v[k] = to_padded ? h[q] : h[2 * p * kPlanePitch + b];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < 2 * PER; ++k) {
-            const uint32_t q = tid + k * kWzpThreads;
-            const uint32_t p = q / blocks, b = q - p * blocks;
-            if (q < halves) (to_padded ? h[2 * p * kPlanePitch + b] : h[q]) = v[k];
-        }
-    }
-}
 
 struct WzpEncodeSmem {
     uint16_t m[kChunk + 8];            // magnitudes (+ slack for word-wide copies)
@@ -116,7 +70,6 @@ struct WzpEncodeSmem {
     uint32_t sgn[kChunk / 32 + 1];     // compacted sign bits (+ slack)
     uint32_t gcount[kChunk / 32];      // nonzero magnitudes per 32-group
     uint32_t gsign[kChunk / 32];       // per 32-group: sign bits of its nonzero magnitudes, compacted
-    uint32_t nsign[kChunk / 32];       // natural sign words of the chunk
     uint32_t sel[16];                  // byte_perm selectors: compact the bytes of a 4-bit mask
     uint8_t pack[256];                 // compressed nibbles: entry 16 * mask + value
     uint32_t tmp[2][kWzpThreads / 32]; // totals of the two block scans
@@ -134,24 +87,6 @@ struct WzpEncodeArgs {
     uint32_t spin_cap;  // lookback wait bound (polls of ~0.2 us)
     uint32_t skip_publish; // test hook: this chunk never publishes (0xffffffff = none)
 };
-
-// 32x32 bit transpose across a warp (five butterfly exchanges): on return
-// lane i holds in bit j what lane j held in bit i. The half-word and byte
-// exchanges are byte permutes; the nibble, pair and bit exchanges are shifts
-// under the stage's mask.
-__device__ __forceinline__ uint32_t warp_transpose32(uint32_t x, int lane) {
-    uint32_t y = __shfl_xor_sync(0xffffffffu, x, 16);
-    x = __byte_perm(x, y, (lane & 16) ? 0x3276u : 0x5410u);
-    y = __shfl_xor_sync(0xffffffffu, x, 8);
-    x = __byte_perm(x, y, (lane & 8) ? 0x3715u : 0x6240u);
-#pragma unroll
-    for (int j = 4; j >= 1; j >>= 1) {
-        const uint32_t m = j == 4 ? 0x0f0f0f0fu : j == 2 ? 0x33333333u : 0x55555555u;
-        y = __shfl_xor_sync(0xffffffffu, x, j);
-        x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y << j) & ~m));
-    }
-    return x;
-}
 
 // Bit 7 of every byte of the result: the byte of w is not zero (other bits 0).
 __device__ __forceinline__ uint32_t nonzero_bytes(uint32_t w) {
@@ -341,23 +276,65 @@ __device__ __forceinline__ uint32_t planes_nonzero(const uint32_t (&w)[8]) {
     return __brev((z | (z >> 16)) & 0xffffu) >> 16;
 }
 
-// Magnitude sources of the encoder. Each fills S.m[0, 8192) (zeros past
-// the chunk's end) and S.nsign (the chunk's natural sign words).
+// One thread per 16-sample block (thread t: Morton slots 16t .. 16t+15 of the
+// chunk): stores the block's packed magnitudes w to S.m, its 16 bit planes to
+// S.planes (full chunks at the padded pitch, a partial chunk in the natural
+// layout, its last count % 16 magnitudes verbatim behind them), and per
+// 32-group the nonzero count and the compacted sign bits of its nonzero
+// magnitudes (the even thread of each pair). nm: negative mask, bit j = slot j
+// (of zero magnitudes: ignored). Slots past the chunk's end hold zero.
+__device__ __forceinline__ void emit_block(WzpEncodeSmem& S, uint32_t (&w)[8], uint32_t nm, uint32_t count, uint32_t t) {
+    const uint32_t blocks = count >> 4;
+    uint4* dm = reinterpret_cast<uint4*>(S.m + 16 * t);
+    dm[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    dm[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    if (t == blocks && (count & 15u)) {
+        uint4* tail = reinterpret_cast<uint4*>(S.planes + 32 * t);
+        tail[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        tail[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+    if ((w[0] | w[1] | w[2] | w[3] | w[4] | w[5] | w[6] | w[7]) != 0) bit_transpose16(w);
+    // group statistics: this block's count and compacted signs, merged with
+    // the odd neighbour's by the even thread of the pair
+    const uint32_t zm = planes_nonzero(w);
+    const uint32_t cnt = __popc(zm), cs = nm ? compress16(nm, zm, S.pack) : 0u;
+    const uint32_t cnt1 = __shfl_xor_sync(0xffffffffu, cnt, 1), cs1 = __shfl_xor_sync(0xffffffffu, cs, 1);
+    if (!(t & 1)) {
+        S.gcount[t >> 1] = cnt + cnt1;
+        S.gsign[t >> 1] = cs | (cs1 << cnt);
+    }
+    if (t < blocks) {
+        uint16_t* pl = reinterpret_cast<uint16_t*>(S.planes);
+        const uint32_t stride = blocks == kChunk / 16 ? 2 * kEncPitch : blocks;
+#pragma unroll
+        for (int p = 0; p < 16; ++p) pl[p * stride + t] = uint16_t(p & 1 ? w[p >> 1] >> 16 : w[p >> 1]);
+    }
+}
+
+// Magnitude sources of the encoder: each fills every block of a chunk through
+// emit_block.
 
 // Morton-packed u16 magnitudes and a natural sign bitmap in global memory.
 struct MagArrays {
-    static constexpr bool kBlockPlanes = false;
     const uint16_t* mag;
     const uint32_t* sign;
-    __device__ __forceinline__ void load(WzpEncodeSmem& S, uint32_t first, uint32_t count, int tid) const {
-        if (count == kChunk) {
-            const uint4* src = reinterpret_cast<const uint4*>(mag + first);
-            for (int i = tid; i < int(kChunk / 8); i += kWzpThreads) reinterpret_cast<uint4*>(S.m)[i] = src[i];
-        } else {
-            for (int i = tid; i < int(kChunk); i += kWzpThreads) S.m[i] = i < int(count) ? mag[first + i] : 0;
+    __device__ __forceinline__ void block_planes(WzpEncodeSmem& S, uint32_t first, uint32_t count, int tid) const {
+        const uint32_t t = uint32_t(tid), at = 16 * t;
+        uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        uint32_t nm = 0;
+        if (at < count) {
+            nm = (sign[(first + at) >> 5] >> (at & 16u)) & 0xffffu;
+            if (at + 16 <= count) {
+                const uint4* src = reinterpret_cast<const uint4*>(mag + first + at);
+                const uint4 a = src[0], b = src[1];
+                w[0] = a.x, w[1] = a.y, w[2] = a.z, w[3] = a.w, w[4] = b.x, w[5] = b.y, w[6] = b.z, w[7] = b.w;
+            } else {
+#pragma unroll
+                for (uint32_t j = 0; j < 16; ++j)
+                    if (at + j < count) w[j >> 1] |= uint32_t(mag[first + at + j]) << (16 * (j & 1u));
+            }
         }
-        for (uint32_t g = tid; g < kChunk / 32; g += kWzpThreads)
-            S.nsign[g] = g * 32 < count ? sign[(first >> 5) + g] : 0u;
+        emit_block(S, w, nm, count, t);
     }
 };
 
@@ -413,7 +390,6 @@ __device__ __forceinline__ uint32_t divide(uint32_t x, uint64_t r, uint32_t d) {
 // rewritten (dequantised) row by row, its magnitudes and negative flags placed
 // at their Morton ranks, and q-outliers recorded as in quantize_kernel.
 template <class T> struct QuantBricks {
-    static constexpr bool kBlockPlanes = true;
     T* coeff;
     uint32_t nx, ny, bz, lb;
     uint64_t rnbx, rnby;  // reciprocals of nx / 16 and ny / 16 (reciprocal())
@@ -496,41 +472,14 @@ template <class T> struct QuantBricks {
         return out;
     }
 
-    // One thread per 16-sample block (thread t: Morton slots 16t .. 16t+15 of
-    // the chunk): quantise the block's four rows (dequantised values written
-    // back), then write its magnitudes to S.m, its 16 bit planes to S.planes
-    // (full chunks at the padded pitch, a partial chunk in the natural
-    // layout), and per 32-group the nonzero count and the compacted sign bits
-    // of its nonzero magnitudes (the even thread of each pair). Blocks past
-    // the chunk's end are zero.
     __device__ __forceinline__ void block_planes(WzpEncodeSmem& S, uint32_t first, uint32_t count, int tid) const {
-        const uint32_t blocks = count >> 4, t = uint32_t(tid);
         uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         uint32_t nm = 0;
-        if (t < blocks) {
-            if (bz == 16) quantise_block<true>(first, t, w, nm);
-            else quantise_block<false>(first, t, w, nm);
+        if (uint32_t(tid) < count >> 4) { // whole bricks: count is a multiple of 16
+            if (bz == 16) quantise_block<true>(first, uint32_t(tid), w, nm);
+            else quantise_block<false>(first, uint32_t(tid), w, nm);
         }
-        uint4* dm = reinterpret_cast<uint4*>(S.m + 16 * t);
-        dm[0] = make_uint4(w[0], w[1], w[2], w[3]);
-        dm[1] = make_uint4(w[4], w[5], w[6], w[7]);
-        if ((w[0] | w[1] | w[2] | w[3] | w[4] | w[5] | w[6] | w[7]) != 0) bit_transpose16(w);
-        // group statistics: this block's count and compacted signs, merged
-        // with the odd neighbour's by the even thread of the pair
-        const uint32_t zm = planes_nonzero(w);
-        const uint32_t cnt = __popc(zm), cs = nm ? compress16(nm, zm, S.pack) : 0u;
-        const uint32_t cnt1 = __shfl_xor_sync(0xffffffffu, cnt, 1), cs1 = __shfl_xor_sync(0xffffffffu, cs, 1);
-        if (!(t & 1)) {
-            S.gcount[t >> 1] = cnt + cnt1;
-            S.gsign[t >> 1] = cs | (cs1 << cnt);
-        }
-        if (t < blocks) {
-            uint16_t* pl = reinterpret_cast<uint16_t*>(S.planes);
-            const bool full = blocks == kChunk / 16;
-            const uint32_t stride = full ? 2 * kEncPitch : blocks;
-#pragma unroll
-            for (int p = 0; p < 16; ++p) pl[p * stride + t] = uint16_t(p & 1 ? w[p >> 1] >> 16 : w[p >> 1]);
-        }
+        emit_block(S, w, nm, count, uint32_t(tid));
     }
 };
 
@@ -554,7 +503,6 @@ __device__ __forceinline__ void WzpEncodeOp<Src>::run(const Params P, uint32_t, 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     WzpEncodeSmem& S = *reinterpret_cast<WzpEncodeSmem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int NW = kWzpThreads / 32;
     const uint32_t chunks = wzp_chunks(A.n), groups = wzp_groups(A.n);
     if (tid == 0) S.chunk = atomicAdd(A.ticket, 1u);
     if (tid < 16) {
@@ -574,75 +522,11 @@ __device__ __forceinline__ void WzpEncodeOp<Src>::run(const Params P, uint32_t, 
     const uint32_t count = min(kChunk, A.n - first);
     const uint32_t blocks = count / 16;
 
-    if constexpr (Src::kBlockPlanes) {
-        // ---- one thread per 16-sample block: magnitudes, bit planes and
-        // group statistics in one pass
-        src.block_planes(S, first, count, tid);
-        for (int i = tid; i < int(kChunk / 32) + 1; i += kWzpThreads) S.sgn[i] = 0;
-        __syncthreads();
-    } else {
-    // ---- magnitudes and natural sign words of the chunk
-    src.load(S, first, count, tid);
+    // ---- one thread per 16-sample block: magnitudes, bit planes and group
+    // statistics in one pass
+    src.block_planes(S, first, count, tid);
     for (int i = tid; i < int(kChunk / 32) + 1; i += kWzpThreads) S.sgn[i] = 0;
     __syncthreads();
-
-    // ---- per 32-group nonzero counts and sign bits, and the bit planes, two
-    // groups per warp step: one 32x32 transpose turns the pair's 16-bit
-    // magnitudes (group g in the high half of each lane's word, g+1 in the
-    // low half) into plane p of g in lane p and of g+1 in lane 16+p
-    const uint32_t in_planes = blocks * 16;
-    for (int k = warp; k < int(kChunk / 64); k += NW) {
-        const int g0 = 2 * k, e0 = g0 * 32 + lane;
-        const uint32_t v = S.m[e0], u = S.m[e0 + 32];
-        const uint32_t nz0 = __ballot_sync(0xffffffffu, v != 0), nz1 = __ballot_sync(0xffffffffu, u != 0);
-        // each group's nonzero magnitudes' sign bits packed in order (merged
-        // at the group's rank below)
-        const uint32_t below = (1u << lane) - 1u;
-        const uint32_t s0 = __reduce_or_sync(
-            0xffffffffu, (v != 0 && ((S.nsign[g0] >> lane) & 1u)) ? 1u << __popc(nz0 & below) : 0u);
-        const uint32_t s1 = __reduce_or_sync(
-            0xffffffffu, (u != 0 && ((S.nsign[g0 + 1] >> lane) & 1u)) ? 1u << __popc(nz1 & below) : 0u);
-        if (lane < 2) {
-            S.gcount[g0 + lane] = __popc(lane ? nz1 : nz0);
-            S.gsign[g0 + lane] = lane ? s1 : s0;
-        }
-        if (uint32_t(g0 * 32) < in_planes) {
-            const uint32_t va = uint32_t(e0) < in_planes ? v : 0u, ua = uint32_t(e0 + 32) < in_planes ? u : 0u;
-            const int top = 32 - __clz(__reduce_or_sync(0xffffffffu, va | ua)); // planes 16-top .. 15 may be set
-            uint32_t mine = 0;
-            if (top > 2) {
-                mine = __brev(warp_transpose32(__brev((va << 16) | ua), lane));
-            } else {
-                // one or two planes: a ballot each (bit 31-e = magnitude e's bit)
-#pragma unroll
-                for (int p = 14; p < 16; ++p) {
-                    if (15 - p < top) {
-                        const uint32_t r0 = __brev(__ballot_sync(0xffffffffu, (va >> (15 - p)) & 1u));
-                        const uint32_t r1 = __brev(__ballot_sync(0xffffffffu, (ua >> (15 - p)) & 1u));
-                        if (lane == p) mine = r0;
-                        if (lane == 16 + p) mine = r1;
-                    }
-                }
-            }
-            // lane l holds plane l % 16 of group g0 + l / 16 (blocks 2g, 2g+1 in
-            // its high and low halves); full chunks: one word at the padded
-            // pitch; a partial chunk keeps the natural layout, u16 words at
-            // p * blocks + b
-            const uint32_t g = uint32_t(g0) + (uint32_t(lane) >> 4), pl_ = uint32_t(lane) & 15u;
-            if (blocks == kChunk / 16) {
-                reinterpret_cast<uint32_t*>(S.planes)[pl_ * kEncPitch + g] = __funnelshift_l(mine, mine, 16);
-            } else {
-                uint16_t* pl = reinterpret_cast<uint16_t*>(S.planes);
-                if (2 * g < blocks) pl[pl_ * blocks + 2 * g] = uint16_t(mine >> 16);
-                if (2 * g + 1 < blocks) pl[pl_ * blocks + 2 * g + 1] = uint16_t(mine & 0xffffu);
-            }
-        }
-    }
-    // verbatim tail after the planes
-    for (uint32_t i = blocks * 16 + tid; i < count; i += kWzpThreads)
-        reinterpret_cast<uint16_t*>(S.planes)[i] = S.m[i];
-    __syncthreads();
-    }
 
     // ---- zero elimination of the plane bytes (thread t owns bytes
     // 32t..32t+31, all of one plane in a warp of a full chunk) and the rank
@@ -839,40 +723,60 @@ struct WzpDirectoryOp {
 struct BrickMap {
     uint32_t nx, ny, nz, bz;
     const uint16_t* local; // 8 slots x 256*bz: rank -> packed brick-local (x | y << 4 | z << 8)
-    const uint16_t* rank;  // 8 slots x 256*bz: brick-local row-major index -> rank (slot 0: whole
-                           // bricks), or null (the decoder then scatters through `local`)
     // Fast map: every brick whole (16 | nx, 16 | ny, bz | nz) and 256*bz a power
     // of two (lb = its log2), so a chunk is a run of whole bricks.
     bool fast;
     uint32_t lb;
+    // Samples of a slab, of a row of bricks (whole / short slab) and of a brick
+    // (short y + 2 * short z), and their reciprocals.
+    uint32_t slab_sz, row_sz[2], brick_sz[4];
+    uint64_t rslab, rrow[2], rbrick[4];
+    static BrickMap make(uint32_t nx, uint32_t ny, uint32_t nz, uint32_t bz, const uint16_t* local) {
+        BrickMap m{};
+        m.nx = nx, m.ny = ny, m.nz = nz, m.bz = bz, m.local = local;
+        const uint32_t bsz = 256 * bz;
+        if (nx % 16 == 0 && ny % 16 == 0 && nz % bz == 0 && (bsz & (bsz - 1)) == 0 && bsz <= kChunk &&
+            kChunk / bsz <= 32) {
+            m.fast = true;
+            while ((1u << m.lb) < bsz) ++m.lb;
+        }
+        // sizes beyond 32 bits divide every index to zero, as the largest does
+        auto fit = [](uint64_t v) { return uint32_t(v < 1 ? 1 : v > 0xffffffffull ? 0xffffffffull : v); };
+        m.slab_sz = fit(uint64_t(nx) * ny * bz);
+        m.rslab = reciprocal(m.slab_sz);
+        for (uint32_t z = 0; z < 2; ++z) {
+            const uint32_t ez = z ? nz % bz : bz;
+            m.row_sz[z] = fit(16ull * nx * ez);
+            m.rrow[z] = reciprocal(m.row_sz[z]);
+            for (uint32_t y = 0; y < 2; ++y) {
+                m.brick_sz[y + 2 * z] = fit(16ull * (y ? ny % 16 : 16) * ez);
+                m.rbrick[y + 2 * z] = reciprocal(m.brick_sz[y + 2 * z]);
+            }
+        }
+        return m;
+    }
     __device__ __forceinline__ uint32_t brick_base(uint32_t b) const {
         const uint32_t nbx = nx / 16, nby = ny / 16;
         const uint32_t bxi = b % nbx, t = b / nbx, byi = t % nby, slab = t / nby;
         return slab * bz * (nx * ny) + byi * 16 * nx + bxi * 16;
     }
-    __device__ __forceinline__ uint32_t in_full_brick(uint32_t base, uint32_t rk) const {
-        const uint32_t loc = __ldg(local + rk);
-        return base + (loc >> 8) * (nx * ny) + ((loc >> 4) & 15u) * nx + (loc & 15u);
-    }
     // Every index fits 32 bits: archives hold at most 2^32 - 1 sample bytes.
+    // Divisions by the host's reciprocals: the hardware has none for integers,
+    // and three per sample were most of this path (181 x 257 x 333 decode of
+    // the stream 0.133 -> 0.080 ms with the block form of the magnitudes).
     __device__ __forceinline__ uint32_t rowmajor(uint32_t k) const {
-        const uint32_t plane = nx * ny;
-        const uint32_t slab_sz = plane * bz;
-        const uint32_t slab = k / slab_sz;
+        const uint32_t slab = divide(k, rslab, slab_sz);
         uint32_t r = k - slab * slab_sz;
-        const uint32_t ez = min(bz, nz - slab * bz);
-        const uint32_t row_sz = 16 * nx * ez;
-        const uint32_t row = r / row_sz;
-        r -= row * row_sz;
-        const uint32_t ey = min(16u, ny - row * 16);
-        const uint32_t brick_sz = 16 * ey * ez;
-        const uint32_t bxi = r / brick_sz;
-        const uint32_t rk = r - bxi * brick_sz;
-        const uint32_t ex = min(16u, nx - bxi * 16);
-        const uint32_t slot = (ex != 16) | ((ey != 16) << 1) | ((ez != bz) << 2);
-        const uint32_t loc = local[slot * 256 * bz + rk];
+        const uint32_t ez = min(bz, nz - slab * bz), pz = ez != bz;
+        const uint32_t row = divide(r, rrow[pz], row_sz[pz]);
+        r -= row * row_sz[pz];
+        const uint32_t ey = min(16u, ny - row * 16), py = ey != 16, at = py + 2 * pz;
+        const uint32_t bxi = divide(r, rbrick[at], brick_sz[at]);
+        const uint32_t rk = r - bxi * brick_sz[at];
+        const uint32_t slot = (nx - bxi * 16 < 16) | (at << 1);
+        const uint32_t loc = __ldg(local + slot * 256 * bz + rk);
         const uint32_t lx = loc & 15, ly = (loc >> 4) & 15, lz = loc >> 8;
-        return (slab * bz + lz) * plane + (row * 16 + ly) * nx + bxi * 16 + lx;
+        return ((slab * bz + lz) * ny + row * 16 + ly) * nx + bxi * 16 + lx;
     }
 };
 
@@ -944,14 +848,11 @@ struct WzpDecodeSmem {
     uint32_t xsel[16];                 // byte_perm selectors: spread 4-bit-mask bytes into place
     uint32_t rep[16];                  // byte_perm selectors: expand repeated bytes
     uint8_t spread[256];               // expanded nibbles: entry 16 * mask + value
-    // full chunks: planes at pitch kEncPitch; a partial chunk: natural, then
-    // repacked to pitch kPlanePitch
-    uint8_t planes[16 * (kEncPitch > kPlanePitch ? kEncPitch : kPlanePitch) * 4];
+    uint8_t planes[16 * kEncPitch * 4]; // full chunks at pitch kEncPitch; a partial chunk: natural
     uint8_t lv[256];                   // level 1 of the repetition elimination
-    uint32_t gprefix[kChunk / 32];
-    uint32_t gmask[kChunk / 32];       // nonzero magnitudes of each 32-group
+    uint32_t nsign[kChunk / 32];       // natural sign words of the decoded magnitudes
     uint32_t tmp[40];
-    uint32_t tmp1[3][kWzpThreads / 32]; // totals of the block scans of whole-brick chunks
+    uint32_t tmp1[3][kWzpThreads / 32]; // totals of the block scans
     uint32_t off, mbytes, sbytes, raw, bad, pos;
 };
 
@@ -1053,7 +954,6 @@ __device__ __forceinline__ void WzpDecodeOp<T>::run(const Params A, uint32_t blo
     extern __shared__ __align__(16) unsigned char smem_raw[];
     WzpDecodeSmem& S = *reinterpret_cast<WzpDecodeSmem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int NW = kWzpThreads / 32;
     const uint32_t chunks = wzp_chunks(A.n), groups = wzp_groups(A.n);
     // block 0 checks the directory beside the chunks' blocks (as a launch of
     // its own it took 4.7 us of every decode)
@@ -1127,7 +1027,7 @@ __device__ __forceinline__ void WzpDecodeOp<T>::run(const Params A, uint32_t blo
     const uint8_t* sgn = S.sb + mis_s;
 
     if (mbytes == 0) {
-        for (int i = tid; i < int(kChunk); i += kWzpThreads) S.m[i] = 0;
+        // nothing stored: every magnitude is zero
     } else if (S.raw) {
         for (int i = tid; i < int(kChunk); i += kWzpThreads)
             S.m[i] = i < int(count) ? uint16_t(gsrc[2 * i] | (gsrc[2 * i + 1] << 8)) : 0;
@@ -1212,160 +1112,72 @@ __device__ __forceinline__ void WzpDecodeOp<T>::run(const Params A, uint32_t blo
             out[0] = make_uint4(words[0], words[1], words[2], words[3]);
             out[1] = make_uint4(words[4], words[5], words[6], words[7]);
         }
-        const bool full = blocks == kChunk / 16;
-        // the verbatim tail (samples past the last whole block) while a
-        // partial chunk's planes are still in the natural layout
-        uint16_t tail = 0;
-        const uint32_t ti = blocks * 16 + tid;
-        if (!full || !blockwise) {
-            __syncthreads();
-            if (ti < count) tail = reinterpret_cast<const uint16_t*>(S.planes)[ti];
-            if (!full) planes_repack(S.planes, blocks, true, tid);
-            __syncthreads();
-        }
-        if (!blockwise) { // else each thread transposes its own block below
-        // ---- inverse bit planes, two groups per warp step: lane l holds plane
-        // l % 16 of group g0 + l / 16 (bit 31-e = magnitude e's bit 15-p); one
-        // 32x32 transpose leaves magnitude e of g0 in the high half of lane e's
-        // word and of g0 + 1 in the low half
-        const uint32_t pitch = full ? kEncPitch : kPlanePitch, in_planes = blocks * 16;
-        for (int k = warp; k < int(kChunk / 64); k += NW) {
-            const int g0 = 2 * k;
-            if (uint32_t(g0 * 32) >= in_planes) break;
-            const uint32_t g = uint32_t(g0) + (uint32_t(lane) >> 4);
-            uint32_t w = 0;
-            if (2 * g < blocks) {
-                const uint32_t word = reinterpret_cast<const uint32_t*>(S.planes)[(uint32_t(lane) & 15u) * pitch + g];
-                w = __funnelshift_l(word, word, 16);
-                if (2 * g + 1 >= blocks) w &= 0xffff0000u;
-            }
-            const uint32_t r = __brev(warp_transpose32(__brev(w), lane));
-            const uint32_t e0 = uint32_t(g0) * 32 + lane, m0 = r >> 16, m1 = r & 0xffffu;
-            if (e0 < in_planes) S.m[e0] = uint16_t(m0);
-            if (e0 + 32 < in_planes) S.m[e0 + 32] = uint16_t(m1);
-            // groups wholly inside the planes: their nonzero counts now
-            const uint32_t nzm0 = __ballot_sync(0xffffffffu, m0 != 0), nzm1 = __ballot_sync(0xffffffffu, m1 != 0);
-            if (lane < 2 && (uint32_t(g0) + lane) * 32 + 32 <= in_planes) {
-                S.gprefix[g0 + lane] = __popc(lane ? nzm1 : nzm0);
-                S.gmask[g0 + lane] = lane ? nzm1 : nzm0;
-            }
-        }
-        for (uint32_t i = blocks * 16 + tid; i < kChunk; i += kWzpThreads)
-            S.m[i] = i == ti ? tail : 0;
-        }
     }
     __syncthreads();
 
-    if (blockwise) {
-        // ---- one thread per 16-sample block (whole bricks): magnitudes from
-        // its 16 bit planes (one transpose) or the verbatim ones, nonzero
-        // ranks by one block scan, signs spread from the sign stream, then the
-        // dequantised block stored as four 16-byte rows
-        const uint32_t t = uint32_t(tid);
-        uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        uint32_t zm = 0; // bit j: magnitude j is not zero
-        if (t < blocks && mbytes != 0) {
-            if (S.raw) {
-                const uint4* sm = reinterpret_cast<const uint4*>(S.m + 16 * t);
-                const uint4 a = sm[0], b = sm[1];
-                w[0] = a.x, w[1] = a.y, w[2] = a.z, w[3] = a.w, w[4] = b.x, w[5] = b.y, w[6] = b.z, w[7] = b.w;
+    // ---- one thread per 16-sample block: magnitudes from its 16 bit planes
+    // (one transpose) or the verbatim ones, nonzero ranks by one block scan,
+    // signs spread from the sign stream
+    const uint32_t t = uint32_t(tid);
+    uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    uint32_t zm = 0; // bit j: magnitude j is not zero
+    if (16 * t < count && mbytes != 0) {
+        if (!S.raw && t < blocks) {
+            const uint16_t* pl = reinterpret_cast<const uint16_t*>(S.planes);
+            const uint32_t stride = blocks == kChunk / 16 ? 2 * kEncPitch : blocks;
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    zm |= (uint32_t((w[i] & 0xffffu) != 0) | (uint32_t((w[i] >> 16) != 0) << 1)) << (2 * i);
-            } else {
-                const uint16_t* pl = reinterpret_cast<const uint16_t*>(S.planes);
-                const uint32_t stride = blocks == kChunk / 16 ? 2 * kEncPitch : 2 * kPlanePitch;
+            for (int i = 0; i < 8; ++i)
+                w[i] = uint32_t(pl[2 * i * stride + t]) | (uint32_t(pl[(2 * i + 1) * stride + t]) << 16);
+            zm = planes_nonzero(w);
+            if (zm) bit_transpose16(w);
+        } else {
+            // a verbatim chunk, or the last count % 16 magnitudes of a partial
+            // one, verbatim behind its planes
+            const uint16_t* sm = S.raw ? S.m : reinterpret_cast<const uint16_t*>(S.planes);
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    w[i] = uint32_t(pl[2 * i * stride + t]) | (uint32_t(pl[(2 * i + 1) * stride + t]) << 16);
-                zm = planes_nonzero(w);
-                if (zm) bit_transpose16(w);
-            }
-        }
-        const uint32_t cnt = __popc(zm);
-        uint32_t nnz;
-        const uint32_t base = block_excl_scan1<kWzpThreads>(cnt, S.tmp1[2], nnz);
-        if (mbytes != 0) {
-            if (nnz == 0 || (nnz + 7) / 8 != sbytes) bad = true;
-            else if ((nnz & 7) && (sgn[sbytes - 1] >> (nnz & 7))) bad = true;
-        }
-        if (t < blocks) {
-            uint32_t nm = 0;
-            if (cnt && !bad) {
-                const uint32_t by = base >> 3;
-                const uint32_t bits = uint32_t(sgn[by]) | (uint32_t(sgn[by + 1]) << 8) | (uint32_t(sgn[by + 2]) << 16);
-                nm = expand16(bits >> (base & 7u), zm, S.spread);
-            }
-            const uint32_t brick = S.bbase[(t << 4) >> A.map.lb];
-            if (A.map.bz == 16) store_block<T, true>(A.map, A.coeff, brick, t, w, nm, q);
-            else store_block<T, false>(A.map, A.coeff, brick, t, w, nm, q);
-        }
-        if (bad) atomicOr(A.status, ST_BAD_STREAM);
-        return;
-    }
-
-    // ---- signs and dequantisation: nonzero counts of the remaining groups
-    const int counted = (mbytes != 0 && !S.raw) ? int(blocks * 16 / 32) : 0;
-    for (int g = counted + warp; g < int(kChunk / 32); g += NW) {
-        const uint32_t nzm = __ballot_sync(0xffffffffu, S.m[g * 32 + lane] != 0);
-        if (lane == 0) {
-            S.gprefix[g] = __popc(nzm);
-            S.gmask[g] = nzm;
+            for (uint32_t j = 0; j < 16; ++j)
+                if (16 * t + j < count) {
+                    const uint32_t m = sm[16 * t + j];
+                    w[j >> 1] |= m << (16 * (j & 1u));
+                    zm |= uint32_t(m != 0) << j;
+                }
         }
     }
-    __syncthreads();
-    uint32_t nnz = 0;
-    {
-        const uint32_t gc = tid < int(kChunk / 32) ? S.gprefix[tid] : 0;
-        const uint32_t gp = block_excl_scan<kWzpThreads>(gc, S.tmp, nnz);
-        if (tid < int(kChunk / 32)) S.gprefix[tid] = gp;
-    }
+    const uint32_t cnt = __popc(zm);
+    uint32_t nnz;
+    const uint32_t base = block_excl_scan1<kWzpThreads>(cnt, S.tmp1[2], nnz);
     if (mbytes != 0) {
         if (nnz == 0 || (nnz + 7) / 8 != sbytes) bad = true;
         else if ((nnz & 7) && (sgn[sbytes - 1] >> (nnz & 7))) bad = true;
     }
-    __syncthreads();
-    // sign of the magnitude at Morton slot e: the sign bit at its rank among
-    // the chunk's nonzero magnitudes
-    auto negative = [&](uint32_t e, uint32_t v) {
-        if (!v || bad) return false;
-        const uint32_t rank = S.gprefix[e >> 5] + __popc(S.gmask[e >> 5] & ((1u << (e & 31u)) - 1u));
-        return rank < 8 * sbytes && ((sgn[rank >> 3] >> (rank & 7)) & 1u);
-    };
-    if (A.map.fast && A.map.rank &&
-        ((reinterpret_cast<uintptr_t>(A.coeff) & 15u) | (reinterpret_cast<uintptr_t>(A.map.rank) & 7u)) == 0) {
-        // whole bricks: four consecutive samples of a brick row per step,
-        // gathered from their Morton slots, one 16-byte store
-        const uint32_t bsz = 1u << A.map.lb, plane = A.map.nx * A.map.ny;
-        for (uint32_t e = 4 * uint32_t(tid); e < count; e += 4 * kWzpThreads) {
-            const uint32_t j = e >> A.map.lb, i = e & (bsz - 1u);
-            const uint32_t at = S.bbase[j] + (i >> 8) * plane + ((i >> 4) & 15u) * A.map.nx + (i & 15u);
-            const uint2 rk = *reinterpret_cast<const uint2*>(A.map.rank + i);
-            T v4[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint32_t slot = (j << A.map.lb) + (((k < 2 ? rk.x : rk.y) >> (16 * (k & 1))) & 0xffffu);
-                const uint32_t v = S.m[slot];
-                const T mag = Lift<T>::mul(T(v), q);
-                v4[k] = negative(slot, v) ? -mag : mag;
-            }
-            store4(A.coeff + at, v4);
-        }
-    } else {
-        for (int g = warp; g < int(kChunk / 32); g += NW) {
-            if (uint32_t(g * 32) >= count) break;
-            const int e = g * 32 + lane;
-            const uint32_t v = S.m[e];
-            if (uint32_t(e) < count) {
-                const T mag = Lift<T>::mul(T(v), q);
-                const uint32_t at = A.map.fast ? A.map.in_full_brick(S.bbase[uint32_t(e) >> A.map.lb],
-                                                                     uint32_t(e) & ((1u << A.map.lb) - 1u))
-                                               : A.map.rowmajor(first + uint32_t(e));
-                A.coeff[at] = negative(uint32_t(e), v) ? -mag : mag;
-            }
-        }
+    uint32_t nm = 0;
+    if (cnt && !bad) {
+        const uint32_t by = base >> 3;
+        const uint32_t bits = uint32_t(sgn[by]) | (uint32_t(sgn[by + 1]) << 8) | (uint32_t(sgn[by + 2]) << 16);
+        nm = expand16(bits >> (base & 7u), zm, S.spread);
     }
     if (bad) atomicOr(A.status, ST_BAD_STREAM);
+    if (blockwise) {
+        // whole bricks: the dequantised block as four 16-byte rows
+        if (t < blocks) {
+            const uint32_t brick = S.bbase[(t << 4) >> A.map.lb];
+            if (A.map.bz == 16) store_block<T, true>(A.map, A.coeff, brick, t, w, nm, q);
+            else store_block<T, false>(A.map, A.coeff, brick, t, w, nm, q);
+        }
+        return;
+    }
+    // ---- edge bricks: 32 consecutive magnitudes per warp step (their samples
+    // share rows), each scattered to its row-major place
+    uint4* dm = reinterpret_cast<uint4*>(S.m + 16 * t);
+    dm[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    dm[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    reinterpret_cast<uint16_t*>(S.nsign)[t] = uint16_t(nm);
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t e = tid; e < count; e += kWzpThreads) {
+        const T mag = Lift<T>::mul(T(uint32_t(S.m[e])), q);
+        A.coeff[A.map.rowmajor(first + e)] = ((S.nsign[e >> 5] >> lane) & 1u) ? -mag : mag;
+    }
 }
 
 } // namespace wb
