@@ -12,6 +12,7 @@ from __future__ import annotations
 import ctypes as C
 import math
 import operator
+from functools import lru_cache
 
 import numpy as np
 
@@ -31,7 +32,11 @@ def _torch():
 
 def _geometry(shape, itemsize):
     """(z,y,x) or (y,x) shape -> (nx, ny, nz), as python/pywaltz/codec.py:24-33."""
-    shape = tuple(operator.index(v) for v in shape)
+    return _dims(tuple(operator.index(v) for v in shape), itemsize)
+
+
+@lru_cache(maxsize=4096)  # a dataset's chunks share a few shapes
+def _dims(shape, itemsize):
     if itemsize not in (4, 8):
         raise TypeError("Waltz requires native float32 or float64")
     if len(shape) not in (2, 3) or min(shape) <= 0:
@@ -48,8 +53,24 @@ def _bound(value):
     return value
 
 
+@lru_cache(maxsize=4096)
 def compressed_capacity(n: int, itemsize: int) -> int:
     return int(lib().waltz_b200_compressed_capacity(n, itemsize))
+
+
+# The batch calls' item structures (Chunk, Archive), filled a column at a time.
+_CHUNK = np.dtype({"names": [f[0] for f in Chunk._fields_], "itemsize": C.sizeof(Chunk),
+                   "formats": ["u8", "u4", "u4", "u4", "f8", "u8", "u8"],
+                   "offsets": [getattr(Chunk, f[0]).offset for f in Chunk._fields_]})
+_ARCHIVE = np.dtype({"names": [f[0] for f in Archive._fields_], "itemsize": C.sizeof(Archive),
+                     "formats": ["u8", "u8", "u8", "u4", "u4", "u4", "u8", "u8", "u8", "u8"],
+                     "offsets": [getattr(Archive, f[0]).offset for f in Archive._fields_]})
+
+
+def _fill_dims(items, shapes, itemsize):
+    dims = np.array([_geometry(s, itemsize) for s in shapes], dtype=np.uint32)
+    for k, name in enumerate(("nx", "ny", "nz")):
+        items[name] = dims[:, k]
 
 
 def _stream(torch, stream):
@@ -148,25 +169,34 @@ def compress_batch(fields, abs_errors, *, out=None, stream=None, tuned=True):
     bounds = [abs_errors] * len(fields) if not hasattr(abs_errors, "__len__") else list(abs_errors)
     if len(bounds) != len(fields):
         raise ValueError("one bound per field")
+    shapes = [tuple(f.shape) for f in fields]
+    caps = [compressed_capacity(math.prod(shape), itemsize) for shape in shapes]
     offsets, total = [], 0
-    for f in fields:
+    for cap in caps:
         total = (total + 15) // 16 * 16
         offsets.append(total)
-        total += compressed_capacity(f.numel(), itemsize)
+        total += cap
     if out is None:
         out = torch.empty(total, dtype=torch.uint8, device=fields[0].device)
     if out.numel() < total or out.dtype != torch.uint8:
         raise ValueError(f"out must be a uint8 CUDA tensor of at least {total} bytes")
-    items = (Chunk * len(fields))()
-    for k, (f, eb, off) in enumerate(zip(fields, bounds, offsets)):
-        nx, ny, nz = _geometry(f.shape, itemsize)
-        items[k] = Chunk(f.data_ptr(), nx, ny, nz, _bound(eb), out.data_ptr() + off,
-                         compressed_capacity(f.numel(), itemsize))
+    items = np.zeros(len(fields), _CHUNK)
+    items["input"] = [f.data_ptr() for f in fields]
+    _fill_dims(items, shapes, itemsize)
+    items["abs_error"] = [_bound(eb) for eb in bounds]
+    items["archive"] = np.array(offsets, dtype=np.uint64) + np.uint64(out.data_ptr())
+    items["capacity"] = caps
     written = (C.c_uint64 * len(fields))()
     if tuned:
-        autotune.apply_batch(lib(), [tuple(f.shape) for f in fields], itemsize)
-    checked(lib().waltz_b200_compress_batch(items, len(fields), itemsize, written, _stream(torch, stream)))
-    return [out[off:off + written[k]] for k, off in enumerate(offsets)]
+        autotune.apply_batch(lib(), shapes, itemsize)
+    checked(lib().waltz_b200_compress_batch((Chunk * len(fields)).from_buffer(items), len(fields), itemsize, written,
+                                            _stream(torch, stream)))
+    # the archives and the gaps between them, in one call
+    pieces, at = [], 0
+    for off, size in zip(offsets, written):
+        pieces += (off - at, size)
+        at = off + size
+    return list(out[:at].split(pieces)[1::2])
 
 
 def decompress_batch(archives, shapes, dtype, *, out=None, headers=None, stream=None, tuned=True):
@@ -202,23 +232,21 @@ def decompress_batch(archives, shapes, dtype, *, out=None, headers=None, stream=
     else:
         if out.dtype != dtype or not out.is_contiguous() or out.numel() < sum(sizes):
             raise ValueError(f"out must be a contiguous {dtype} tensor of at least {sum(sizes)} samples")
-        flat, views, at = out.view(-1), [], 0
-        for k, s in zip(sizes, shapes):
-            views.append(flat[at:at + k].view(s))
-            at += k
-    keep = []
-    items = (Archive * len(archives))()
-    for k, (a, s, v) in enumerate(zip(archives, shapes, views)):
-        nx, ny, nz = _geometry(s, itemsize)
-        hdr = None
-        if headers is not None:
-            buf = C.create_string_buffer(bytes(headers[k][:32]), 32)
-            keep.append(buf)
-            hdr = C.cast(buf, C.c_void_p)
-        items[k] = Archive(a.data_ptr(), a.numel(), hdr, nx, ny, nz, v.data_ptr(), v.numel() * itemsize)
+        views = [v.view(s) for v, s in zip(out.view(-1)[:sum(sizes)].split(sizes), shapes)]
+    items = np.zeros(len(archives), _ARCHIVE)
+    items["archive"] = [a.data_ptr() for a in archives]
+    items["bytes"] = [a.numel() for a in archives]
+    if headers is not None:
+        heads = np.frombuffer(b"".join(bytes(headers[k][:32]).ljust(32, b"\0") for k in range(len(archives))),
+                              dtype=np.uint8)
+        items["header"] = heads.ctypes.data + 32 * np.arange(len(archives), dtype=np.uint64)
+    _fill_dims(items, shapes, itemsize)
+    items["output"] = [v.data_ptr() for v in views]
+    items["output_bytes"] = [k * itemsize for k in sizes]
     if tuned:
         autotune.apply_batch(lib(), shapes, itemsize)
-    checked(lib().waltz_b200_decompress_batch(items, len(archives), itemsize, _stream(torch, stream)))
+    checked(lib().waltz_b200_decompress_batch((Archive * len(archives)).from_buffer(items), len(archives), itemsize,
+                                              _stream(torch, stream)))
     return views
 
 
