@@ -11,7 +11,7 @@ from tests.test_gpu_parity import gpu_compress, gpu_decompress, gpu_transform
 
 pytestmark = pytest.mark.gpu
 
-# (nx, ny, nz), dyadic. Strips of 32 x start at 4 mod 32, Z windows hold 16
+# (nx, ny, nz), dyadic. Strips of 32 x start at 28 mod 32, Z windows hold 16
 # planes, Y windows 8 rows; the finest level's half row is a multiple of 4
 # (the staged kernels) except in the last two (the register marches).
 LEVEL_SHAPES = [(24, 9, 9), (40, 15, 16), (24, 17, 15), (72, 31, 17), (32, 40, 23), (136, 33, 34), (64, 65, 66),

@@ -10,7 +10,7 @@
 // rows (3.4 cells staged per output), a step stages 1.9 cells per output and
 // lifts 1.9 along Z and 1.25 along X; the boxes of the next step land in the
 // other buffer meanwhile.
-//  * The strips start at 4 mod 32, so a footprint's first coefficient is a
+//  * The strips start at 28 mod 32, so a footprint's first coefficient is a
 //    multiple of 4 (the copy engine's 16-byte rule) without padding columns,
 //    and box rows of 20 floats put the eight 16-byte accesses of a quarter
 //    warp in distinct banks. X does not fold, so any strip origin gives the
@@ -33,33 +33,6 @@
 #include "tma.cuh"
 
 namespace wb {
-
-// lift_inverse<float, P, true> (common.cuh) on two lines at once.
-template <int P> __device__ __forceinline__ void lift_inverse2(f2 (&e)[P], f2 (&o)[P]) {
-    const f2 ca = f2_pack(-K97<float>::a, -K97<float>::a), cb = f2_pack(-K97<float>::b, -K97<float>::b),
-             cg = f2_pack(-K97<float>::g, -K97<float>::g), cd = f2_pack(-K97<float>::d, -K97<float>::d),
-             ck = f2_pack(-K97<float>::k, -K97<float>::k), ci = f2_pack(K97<float>::ik, K97<float>::ik);
-    const f2 raw_first = o[0], raw_last = o[P - 1];
-#pragma unroll
-    for (int j = 0; j < P; ++j) {
-        e[j] = f2_mul(e[j], ci);
-        o[j] = f2_mul(o[j], ck);
-    }
-#pragma unroll
-    for (int j = 1; j < P; ++j) {
-        f2 s;
-        if (j == 1) s = f2_fma(raw_first, ck, o[1]);
-        else if (j == P - 1) s = f2_fma(raw_last, ck, o[P - 2]);
-        else s = f2_add(o[j - 1], o[j]);
-        e[j] = f2_fma(cd, s, e[j]);
-    }
-#pragma unroll
-    for (int j = 1; j < P - 1; ++j) o[j] = f2_fma(cg, f2_add(e[j], e[j + 1]), o[j]);
-#pragma unroll
-    for (int j = 2; j < P - 1; ++j) e[j] = f2_fma(cb, f2_add(o[j - 1], o[j]), e[j]);
-#pragma unroll
-    for (int j = 2; j < P - 2; ++j) o[j] = f2_fma(ca, f2_add(e[j], e[j + 1]), o[j]);
-}
 
 // Emitters that store at base + z * sz + y * sy + x, with the status word of
 // their finiteness check (null: none).
@@ -89,7 +62,7 @@ template <class T> struct LinearOut<JobOut<T>> {
 
 struct InvMarch {
     static constexpr int UX = 32, UZ = 16, UY = 8;    // outputs of a step
-    static constexpr int SHIFT = 28;                  // strip b covers x = 32 b - 28 .. 32 b + 3
+    static constexpr int SHIFT = 4;                   // strip b covers x = 32 b - 4 .. 32 b + 27
     static constexpr int HX = UX / 2 + 4, HY = UY / 2, HZ = UZ / 2 + 4;
     static constexpr int BOX = HZ * HY * HX;          // floats per parity box
     static constexpr int STAGE = 8 * BOX;             // floats per step
@@ -258,7 +231,7 @@ __device__ __forceinline__ void InvMarchOp<Out>::run(const Params& P, uint32_t b
         if constexpr (Out::kPrefetch) {
             if (t > 0 && tid < S::UY * S::UZ) {
                 const uint32_t gy = uint32_t(r0 - 4 + tid % S::UY), gz = uint32_t(oz + tid / S::UY);
-                if (gy < a.y && gz < a.z) out.warm(uint32_t(max(ox, 0)), gy, gz);
+                if (gy < a.y && gz < a.z) out.warm(min(uint32_t(ox + S::SHIFT), a.x - 1), gy, gz); // most of the row
             }
         }
         // a copy that never lands: the status fails the call, and the later

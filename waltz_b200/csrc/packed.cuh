@@ -37,4 +37,31 @@ __device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
     return r;
 }
 
+// lift_inverse<float, P, true> (common.cuh) on two lines at once.
+template <int P> __device__ __forceinline__ void lift_inverse2(f2 (&e)[P], f2 (&o)[P]) {
+    const f2 ca = f2_pack(-K97<float>::a, -K97<float>::a), cb = f2_pack(-K97<float>::b, -K97<float>::b),
+             cg = f2_pack(-K97<float>::g, -K97<float>::g), cd = f2_pack(-K97<float>::d, -K97<float>::d),
+             ck = f2_pack(-K97<float>::k, -K97<float>::k), ci = f2_pack(K97<float>::ik, K97<float>::ik);
+    const f2 raw_first = o[0], raw_last = o[P - 1];
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+        e[j] = f2_mul(e[j], ci);
+        o[j] = f2_mul(o[j], ck);
+    }
+#pragma unroll
+    for (int j = 1; j < P; ++j) {
+        f2 s;
+        if (j == 1) s = f2_fma(raw_first, ck, o[1]);
+        else if (j == P - 1) s = f2_fma(raw_last, ck, o[P - 2]);
+        else s = f2_add(o[j - 1], o[j]);
+        e[j] = f2_fma(cd, s, e[j]);
+    }
+#pragma unroll
+    for (int j = 1; j < P - 1; ++j) o[j] = f2_fma(cg, f2_add(e[j], e[j + 1]), o[j]);
+#pragma unroll
+    for (int j = 2; j < P - 1; ++j) e[j] = f2_fma(cb, f2_add(o[j - 1], o[j]), e[j]);
+#pragma unroll
+    for (int j = 2; j < P - 2; ++j) o[j] = f2_fma(ca, f2_add(e[j], e[j + 1]), o[j]);
+}
+
 } // namespace wb

@@ -25,6 +25,7 @@
 // pairs of rows shared with the next window stay in registers); nothing is
 // staged in shared memory.
 #pragma once
+#include "packed.cuh"
 #include "transform.cuh"
 
 namespace wb {
@@ -230,16 +231,28 @@ __device__ __forceinline__ void XYMarchOp<T, Inverse, Src, Out>::run(const Param
                 pre[k][1] = (live_o && y0 + k < a.y) ? out.fetch(uint32_t(xe) + 1, y0 + k, z) : T(0);
             }
         }
+        if constexpr (Inverse && sizeof(T) == 4) {
+            // both columns of the pair along Y at once, in packed registers
+            // (181 x 257 x 333 finest level 0.077 -> 0.075 ms; the forward
+            // march, whose rows go on to the shuffles, lost 7 % with it)
+            f2 ye[PP], yo[PP];
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            // one column of the pair along Y, in registers
-            T ye[PP], yo[PP];
+            for (int j = 0; j < PP; ++j) ye[j] = f2_pack(e[j][0], e[j][1]), yo[j] = f2_pack(o[j][0], o[j][1]);
+            lift_inverse2<PP>(ye, yo);
 #pragma unroll
-            for (int j = 0; j < PP; ++j) ye[j] = e[j][c], yo[j] = o[j][c];
-            if constexpr (Inverse) lift_inverse<T, PP, true>(ye, yo);
-            else lift_forward<T, PP>(ye, yo);
+            for (int j = 0; j < PP; ++j) f2_unpack(ye[j], e[j][0], e[j][1]), f2_unpack(yo[j], o[j][0], o[j][1]);
+        } else {
 #pragma unroll
-            for (int j = 0; j < PP; ++j) e[j][c] = ye[j], o[j][c] = yo[j];
+            for (int c = 0; c < 2; ++c) {
+                // one column of the pair along Y, in registers
+                T ye[PP], yo[PP];
+#pragma unroll
+                for (int j = 0; j < PP; ++j) ye[j] = e[j][c], yo[j] = o[j][c];
+                if constexpr (Inverse) lift_inverse<T, PP, true>(ye, yo);
+                else lift_forward<T, PP>(ye, yo);
+#pragma unroll
+                for (int j = 0; j < PP; ++j) e[j][c] = ye[j], o[j][c] = yo[j];
+            }
         }
         const uint32_t x = uint32_t(xe);
 #pragma unroll

@@ -110,6 +110,7 @@ template <class T> struct ZmStore {
     template <class V>
     __device__ __forceinline__ void group(uint32_t col, uint32_t z0, uint32_t nz, size_t ncols,
                                           const V (&r)[16]) const {
+        if (col >= ncols) return;
 #pragma unroll
         for (int j = 0; j < 16; ++j)
             if (z0 + j < nz) dst[size_t(z0 + j) * ncols + col] = T(r[j]);
@@ -119,18 +120,28 @@ template <class T, class Final> struct ZmEmit {
     Final fin;
     uint32_t nx;
     template <class V>
-    __device__ __forceinline__ void group(uint32_t col, uint32_t z0, uint32_t nz, size_t, const V (&r)[16]) const {
-        const uint32_t x = col % nx, y = col / nx;
+    __device__ __forceinline__ void group(uint32_t col, uint32_t z0, uint32_t nz, size_t ncols, const V (&r)[16]) const {
         if constexpr (Final::kPrefetch) {
             // every original first, then the emissions: the loads do not wait
-            // behind the emitter's stores
+            // behind the emitter's stores. The field is dense, so a warp's 32
+            // columns are 32 consecutive samples of every plane; lane j keeps
+            // the patched mask of plane z0 + j
+            const bool live = col < ncols;
+            const uint32_t lane = threadIdx.x & 31u;
             T o[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) o[j] = z0 + j < nz ? fin.fetch(x, y, z0 + j) : T(0);
+            for (int j = 0; j < 16; ++j) o[j] = (live && z0 + j < nz) ? __ldg(fin.orig + size_t(z0 + j) * ncols + col) : T(0);
+            uint32_t mine = 0;
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-                if (z0 + j < nz) fin.emit(x, y, z0 + j, T(r[j]), o[j]);
+            for (int j = 0; j < 16; ++j) {
+                if (z0 + j >= nz) break;
+                const uint32_t m = fin.emit_row(T(r[j]), o[j], size_t(z0 + j) * ncols + col, live);
+                if (lane == uint32_t(j)) mine = m;
+            }
+            if (mine) fin.put_row(int64_t(size_t(z0 + lane) * ncols) + int64_t(col) - lane, mine);
         } else {
+            if (col >= ncols) return;
+            const uint32_t x = col % nx, y = col / nx;
 #pragma unroll
             for (int j = 0; j < 16; ++j)
                 if (z0 + j < nz) fin(x, y, z0 + j, T(r[j]));
@@ -265,7 +276,7 @@ __global__ void __launch_bounds__(kZmThreads, 2)
             float f[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(r[j]);
-            if (col < ncols) out.group(uint32_t(col), c0, nz, ncols, f);
+            out.group(uint32_t(col), c0, nz, ncols, f);
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads(); // tensor memory read out: the next tile's MMAs may overwrite it
@@ -442,7 +453,7 @@ __global__ void __launch_bounds__(kZmThreads, 2)
                 float f[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(r[j]);
-                if (ocol < ncols) out.group(uint32_t(ocol), c0, nz, ncols, f);
+                out.group(uint32_t(ocol), c0, nz, ncols, f);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncthreads(); // tensor memory read out: the next tile's MMAs may overwrite it
@@ -689,7 +700,7 @@ __global__ void __launch_bounds__(kZmThreads, 2)
             float f[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(r[j]);
-            if (ocol < ncols) out.group(uint32_t(ocol), c0, nz, ncols, f);
+            out.group(uint32_t(ocol), c0, nz, ncols, f);
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads(); // tensor memory read out: the next tile's MMAs may overwrite it
@@ -817,7 +828,7 @@ __global__ void __launch_bounds__(kZmThreads, 2)
             }
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = v[j] * cs * (c0 + j < P.np ? bscale[c0 + j] : 0.0);
-            if (ocol < ncols) out.group(uint32_t(ocol), c0, nz, ncols, v);
+            out.group(uint32_t(ocol), c0, nz, ncols, v);
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads(); // tensor memory read out: the next tile's MMAs may overwrite it
