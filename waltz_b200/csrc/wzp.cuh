@@ -946,11 +946,13 @@ template <class T> struct WzpDecodeArgs {
 template <class T> struct WzpDecodeOp {
     static constexpr int kThreads = kWzpThreads, kMinBlocks = 4; // 32 registers: four CTAs per SM
     using Params = WzpDecodeArgs<T>;
-    static __device__ __forceinline__ void run(const Params A, uint32_t block, uint32_t);
+    // by reference: the brick map is indexed, which would put a batch's copy of
+    // the parameters into local memory
+    static __device__ __forceinline__ void run(const Params& A, uint32_t block, uint32_t);
 };
 
 template <class T>
-__device__ __forceinline__ void WzpDecodeOp<T>::run(const Params A, uint32_t block, uint32_t) {
+__device__ __forceinline__ void WzpDecodeOp<T>::run(const Params& A, uint32_t block, uint32_t) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     WzpDecodeSmem& S = *reinterpret_cast<WzpDecodeSmem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
