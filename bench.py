@@ -910,11 +910,11 @@ def batch_only(dev, lib, args, count=512):
 # (profiles/dram_traffic_f32_512cubed_rel1e-3.md). A run on another shape
 # reports no traffic.
 TRAFFIC_512 = {
-    "compress:fwd_l0": 1045993984,
-    "compress:wzp_encode": 1110756608,
-    "compress:inv_l0_repair": 1309071616,
-    "decompress:wzp_decode": 576808704,
-    "decompress:inv_l0": 1053336576,
+    "compress:fwd_l0": 1042545408,
+    "compress:wzp_encode": 1107133440,
+    "compress:inv_l0_repair": 1320829240,
+    "decompress:wzp_decode": 572814336,
+    "decompress:inv_l0": 1069107200,
 }
 
 

@@ -121,12 +121,12 @@ int waltz_b200_decompress_batch(const waltz_b200_archive* archives, uint32_t cou
  * WALTZ_B200_OPT_ZMARCH_PLANES (0 = automatic, else >= 16): planes per CTA of
  *   the forward dyadic z-march (work per tile against the 8-plane halo).
  * WALTZ_B200_OPT_SMALL_LEVEL (samples, default 2^15, 0 = none): inverse
- *   levels (dyadic, and the plane schedule's XY levels) of at most this many
- *   samples stage their tiles with reflecting loads instead of tensor-map
- *   copies (their tiles are almost all edge tiles).
+ *   levels of at most this many samples (the plane schedule's XY levels, and
+ *   dyadic levels of doubles) run as register marches instead of tiles staged
+ *   by tensor-map copies. Float dyadic levels always take the staged y-march,
+ *   and rows the copy engine cannot stage always take the register marches.
  * WALTZ_B200_OPT_SMALL_FWD (samples, default 2^20, 0 = none): the same for
- *   forward levels (dyadic and XY), whose z-march may then also use 8-plane
- *   ranges. */
+ *   forward levels (dyadic and XY, both types). */
 #define WALTZ_B200_OPT_STAGE_KERNELS 1
 #define WALTZ_B200_OPT_ZMARCH_PLANES 2
 #define WALTZ_B200_OPT_SMALL_LEVEL 3
@@ -151,7 +151,7 @@ int waltz_b200_decompress_batch(const waltz_b200_archive* archives, uint32_t cou
  *   change. */
 #define WALTZ_B200_OPT_XY_MARCH 6
 /* WALTZ_B200_OPT_SMALL_MARCH (samples, default 0 = none): dyadic inverse
- *   levels of at most this many samples run as two register marches (the Z
+ *   levels of doubles of at most this many samples run as two register marches (the Z
  *   synthesis, then the X and Y synthesis) instead of the tile inverse, whose
  *   tiles cannot fill the GPU on small levels. A performance knob like the
  *   others: the bytes do not change. */

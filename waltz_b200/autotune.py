@@ -6,9 +6,9 @@ question and the table can be applied blindly):
  * single fields: the plane schedule's whole-stage kernels on or off
    (WALTZ_B200_OPT_STAGE_KERNELS), the forward z-march depth, the planes
    per CTA tile of the dyadic forward levels (WALTZ_B200_OPT_ZMARCH_PLANES),
-   and the level sizes below which dyadic and XY levels stage tiles with
-   reflecting loads instead of tensor-map copies (WALTZ_B200_OPT_SMALL_LEVEL /
-   _FWD);
+   and the level sizes below which dyadic and XY levels run as register
+   marches instead of tiles staged by tensor-map copies
+   (WALTZ_B200_OPT_SMALL_LEVEL / _FWD);
  * batches: the execution form of the batch graph (stage-batched groups,
    the same as persistent work queues, or per-field chains, and their width,
    waltz_b200_batch_config), the stage kernels knob and, for stage-batched
@@ -17,8 +17,9 @@ question and the table can be applied blindly):
    level (the small-level thresholds at 0) and the plane XY levels as the
    warp march, forward and inverse levels separately
    (WALTZ_B200_OPT_XY_MARCH bits 0 and 1; single plane fields try it too),
-   and the size up to which dyadic inverse levels run as a Z march and an
-   XY march instead of the tile inverse (WALTZ_B200_OPT_SMALL_MARCH), and
+   and the size up to which dyadic inverse levels of doubles run as a Z march
+   and an XY march instead of the tile inverse (WALTZ_B200_OPT_SMALL_MARCH;
+   float levels take the y-march at every size), and
    dyadic forward levels as an XY march and a Z march instead of the
    z-march (WALTZ_B200_OPT_SMALL_MARCH_FWD); single dyadic fields try both;
  * the transform form (lifting or one split of the tensor-core matrix form)

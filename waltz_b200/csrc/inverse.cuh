@@ -1,4 +1,6 @@
-// Inverse dyadic level (synthesis Z, X, Y) from TMA-staged parity boxes.
+// Inverse dyadic level of a double field (synthesis Z, X, Y) from TMA-staged
+// parity boxes (float levels take the y-march of invmarch.cuh, which keeps the
+// box scheme described here).
 //
 // The coefficients of one level live in the reference's split-band layout:
 // along each axis the even spatial positions are the low half [0, ceil(n/2))
@@ -28,9 +30,6 @@
 namespace wb {
 
 template <class T> struct InvTile;
-template <> struct InvTile<float> {
-    static constexpr int UX = 32, UY = 16, UZ = 16;
-};
 template <> struct InvTile<double> {
     static constexpr int UX = 16, UY = 16, UZ = 8;
 };
@@ -57,9 +56,7 @@ template <class T> struct InvLevel {
 };
 
 template <class T, int UX, int UY, int UZ, class Out> struct InvTileOp {
-    // float tiles: 16 warps per CTA, two CTAs per SM (the passes have 512 to
-    // 960 items); double tiles are half as wide and keep 8 warps
-    static constexpr int kThreads = sizeof(T) == 4 ? 512 : 256, kMinBlocks = 2;
+    static constexpr int kThreads = 256, kMinBlocks = 2;
     static constexpr bool kGridConstant = true;
     struct Params {
         CUtensorMap cmap, lmap;

@@ -384,11 +384,11 @@ __device__ __forceinline__ uint32_t divide(uint32_t x, uint64_t r, uint32_t d) {
     return d > 1 ? uint32_t(__umul64hi(uint64_t(x), r)) : x;
 }
 
-// The coefficients themselves, quantised by the encoder (quantize_kernel
-// fused in): the chunk is a run of whole 16 x 16 x bz bricks (2^lb samples
+// The coefficients themselves, quantised by the encoder (QuantizeOp fused
+// in): the chunk is a run of whole 16 x 16 x bz bricks (2^lb samples
 // each, the field made of whole bricks only); every brick is read and
 // rewritten (dequantised) row by row, its magnitudes and negative flags placed
-// at their Morton ranks, and q-outliers recorded as in quantize_kernel.
+// at their Morton ranks, and q-outliers recorded as in QuantizeOp.
 template <class T> struct QuantBricks {
     T* coeff;
     uint32_t nx, ny, bz, lb;
