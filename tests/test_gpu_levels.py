@@ -48,3 +48,20 @@ def test_extrema_at_any_alignment(n, offset, dtype):
         a[offset], a[offset + 1] = np.nan, -np.inf
         view = torch.from_numpy(a).cuda()[offset:]
         assert waltz_b200.extrema(view) == (-np.inf, float(np.nanmax(a[offset:])))
+
+
+@pytest.mark.parametrize("form", ["matrix-tf32", "matrix-bf16", "matrix-exact"])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_matrix_repairs_with_a_partial_last_warp(form, dtype):
+    """612 columns: the last warp of the matrix synthesis holds four of them.
+    Every sample meets the bound and the decode repeats."""
+    import waltz_b200
+    from waltz_b200 import synthetic as S
+    a = S.power_law_field((33, 18, 34), 6, dtype=dtype)
+    eb = float(np.float32(1e-3))
+    archive = waltz_b200.compress(a, abs_error=eb, form=form)
+    assert int.from_bytes(archive[24:28], "little") > 0, "the field has repairs"
+    out = waltz_b200.decompress(archive, shape=a.shape, dtype=dtype)
+    assert np.abs(out.astype(np.float64) - a.astype(np.float64)).max() <= eb
+    assert waltz_b200.decompress(archive, shape=a.shape, dtype=dtype).tobytes() == out.tobytes()
+    assert waltz_b200.compress(a, abs_error=eb, form=form) == archive
