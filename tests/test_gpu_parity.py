@@ -371,6 +371,22 @@ def test_matrix_form_round_trip_float64(shape, eb):
     assert err <= np.longdouble(eb)
 
 
+@pytest.mark.parametrize("nxyz", [(48, 32, 16), (37, 33, 17)])  # whole bricks; edge bricks
+@pytest.mark.parametrize("sign", [1, -1])
+def test_codes_at_the_top_of_the_fast_rounding(nxyz, sign):
+    """Scaled float coefficients on both sides of 2^22, where the one-add
+    rounding ends: 4194303.5 and above round to 4194304, with their sign."""
+    rng = np.random.default_rng(1)
+    a = (sign * (1.0 + 3e-6 * rng.standard_normal(P.zyx(nxyz)))).astype(np.float32)
+    c = sign * O.transform(a, inverse=False)
+    eb = float(np.median(c[c > 0.9 * c.max()])) / (1.5 * 4194303.6)
+    scaled = c * np.float32(1.0 / (1.5 * eb))
+    assert np.isin(scaled, np.float32([4194303.5, 4194303.75])).sum() > 10 and (scaled == 4194304.5).any()
+    expect = O.compress(a, eb)
+    assert gpu_compress(a, eb) == expect
+    assert gpu_decompress(expect, a.shape, a.dtype).tobytes() == O.decompress(expect, a.shape, a.dtype).tobytes()
+
+
 BATCH_FORMS = [(0, 1), (0, 3), (1, 32), (2, 1), (2, 4)]  # (stage-batched | field chains | work queue, width)
 
 

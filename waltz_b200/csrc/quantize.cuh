@@ -35,16 +35,18 @@ template <class T> struct QuantArgs {
 
 constexpr int kQuantThreads = 256;
 
-// Rounds x (|x| below kFastQuant) to the nearest integer, ties to even,
-// with one add of 1.5 * 2^(mantissa bits): the sum's low bits then hold the
-// rounded value. Returns the integer; `back` receives it as T exactly.
+// Rounds x (|x| below kLimit) to the nearest integer, ties to even, with one
+// add of 1.5 * 2^(mantissa bits): the sum's bits less the constant's are then
+// the rounded value. Returns the integer; `back` receives it as T exactly.
 template <class T> struct FastRound;
 template <> struct FastRound<float> {
     static constexpr float kLimit = 4194304.0f; // 2^22
     static __device__ __forceinline__ int32_t round(float x, float& back) {
         const float t = __fadd_rn(x, 12582912.0f); // 1.5 * 2^23
         back = __fsub_rn(t, 12582912.0f);
-        return int32_t(__float_as_uint(t) & 0x7fffffu) - 0x400000;
+        // the difference of the whole words: from 4194303.5 on the sum rounds
+        // up to 2^24, the next binade, whose mantissa bits alone are zero
+        return int32_t(__float_as_uint(t) - 0x4b400000u);
     }
 };
 template <> struct FastRound<double> {
