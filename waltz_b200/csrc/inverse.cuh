@@ -397,6 +397,7 @@ __device__ __forceinline__ void InvTileXYOp<T, UX, UY, UZ, Out>::run(const Param
                         y0 + (yp ? int(hy) : 0), int(oz), bar);
         }
     }
+    __syncwarp(); // the barrier is initialised before the other lanes of warp 0 poll it
     {
         const bool ok = __syncthreads_and(warp != 0 || mbar_wait(bar, 0, kWaitBound));
         if (!ok) {
