@@ -430,6 +430,35 @@ def test_batch_compress_equals_single_calls(batch_form):
         waltz_b200.compress_batch(bad, 1e-3)
 
 
+@pytest.mark.parametrize("shape", [(64, 64, 64), (24, 96, 64)])  # dyadic; plane schedule
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_work_queue_items_reuse_the_staged_buffers(dtype, shape):
+    """A work queue whose CTAs take several items of the staged levels each
+    (128 equal fields, about 400 resident CTAs, every level staged by tensor
+    copies): archives and decodes are those of the single-field calls."""
+    torch = _torch()
+    import waltz_b200
+    from waltz_b200 import autotune as A
+    from waltz_b200 import synthetic as S
+    lib = _lib()
+    base = [torch.from_numpy(S.power_law_field(shape, 60 + k).astype(dtype)).cuda() for k in range(4)]
+    fields = [base[k % 4] * (1.0 + k / 7) for k in range(128)]
+    bounds = [float(np.float32(2e-3 * float(f.max() - f.min()))) for f in fields]
+    singles = [waltz_b200.compress_tensor(f, eb) for f, eb in zip(fields, bounds)]
+    decoded = [waltz_b200.decompress_tensor(a, shape, base[0].dtype) for a in singles]
+    assert bytes(singles[0].cpu().numpy()) == O.compress(fields[0].cpu().numpy(), bounds[0])
+    try:
+        assert lib.waltz_b200_batch_config(2, 1) == 0
+        A.set_single(lib, {"stage_kernels": 0, "small_inv": 0, "small_fwd": 0})
+        archives = waltz_b200.compress_batch(fields, bounds, tuned=False)
+        assert all(torch.equal(a, r) for a, r in zip(archives, singles))
+        out = waltz_b200.decompress_batch(archives, [shape] * 128, base[0].dtype, tuned=False)
+        assert all(torch.equal(a, r) for a, r in zip(out, decoded))
+    finally:
+        A.set_single(lib, {})
+        lib.waltz_b200_batch_config(1, 32)
+
+
 def _uneven_batch(torch, seed, count, sides=(16, 17, 32, 48, 64)):
     from waltz_b200 import synthetic as S
     rng = np.random.default_rng(seed)

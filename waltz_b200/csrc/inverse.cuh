@@ -70,6 +70,14 @@ template <class T, int UX, int UY, int UZ, class Out> struct InvTileOp {
         tensormap_acquire(&P.cmap);
         if (P.lv.low) tensormap_acquire(&P.lmap);
     }
+    static constexpr int kBarriers = 4;
+    static __device__ __forceinline__ T* staged() { // the parity boxes
+        extern __shared__ __align__(128) unsigned char inv_smem[];
+        return reinterpret_cast<T*>(inv_smem + ((128 - (smem_u32(inv_smem) & 127)) & 127));
+    }
+    static __device__ __forceinline__ uint64_t* barriers() {
+        return reinterpret_cast<uint64_t*>(staged() + 8 * InvShape<T, UX, UY, UZ>::BOX);
+    }
 };
 
 template <class T, int UX, int UY, int UZ, class Out>
@@ -79,9 +87,8 @@ __device__ __forceinline__ void InvTileOp<T, UX, UY, UZ, Out>::run(const Params&
     const Out out = P.out;
     uint32_t* const status = P.status;
     using S = InvShape<T, UX, UY, UZ>;
-    extern __shared__ __align__(128) unsigned char inv_smem[];
-    T* Bx = reinterpret_cast<T*>(inv_smem + ((128 - (smem_u32(inv_smem) & 127)) & 127));
-    uint64_t* bar = reinterpret_cast<uint64_t*>(Bx + 8 * S::BOX);
+    T* Bx = staged();
+    uint64_t* bar = barriers();
     const int tid = threadIdx.x, warp = tid >> 5;
     const Dims a = lv.a;
     const uint32_t bx = block % tiles_x, by = (block / tiles_x) % tiles_y, bz = block / (tiles_x * tiles_y);
@@ -359,6 +366,14 @@ template <class T, int UX, int UY, int UZ, class Out> struct InvTileXYOp {
         tensormap_acquire(&P.cmap);
         if (P.lv.low) tensormap_acquire(&P.lmap);
     }
+    static constexpr int kBarriers = 1;
+    static __device__ __forceinline__ T* staged() { // the parity boxes
+        extern __shared__ __align__(128) unsigned char inv_smem[];
+        return reinterpret_cast<T*>(inv_smem + ((128 - (smem_u32(inv_smem) & 127)) & 127));
+    }
+    static __device__ __forceinline__ uint64_t* barriers() {
+        return reinterpret_cast<uint64_t*>(staged() + 4 * InvXYShape<T, UX, UY, UZ>::BOX);
+    }
 };
 
 template <class T, int UX, int UY, int UZ, class Out>
@@ -368,9 +383,8 @@ __device__ __forceinline__ void InvTileXYOp<T, UX, UY, UZ, Out>::run(const Param
     const Out out = P.out;
     uint32_t* const status = P.status;
     using S = InvXYShape<T, UX, UY, UZ>;
-    extern __shared__ __align__(128) unsigned char inv_smem[];
-    T* Bx = reinterpret_cast<T*>(inv_smem + ((128 - (smem_u32(inv_smem) & 127)) & 127));
-    uint64_t* bar = reinterpret_cast<uint64_t*>(Bx + 4 * S::BOX);
+    T* Bx = staged();
+    uint64_t* bar = barriers();
     const int tid = threadIdx.x, warp = tid >> 5;
     const Dims a = lv.a;
     const uint32_t bx = block % tiles_x, by = (block / tiles_x) % tiles_y, bz = block / (tiles_x * tiles_y);

@@ -88,6 +88,14 @@ template <class Out> struct InvMarchOp {
         tensormap_acquire(&P.cmap);
         if (P.lv.low) tensormap_acquire(&P.lmap);
     }
+    static constexpr int kBarriers = 2;
+    static __device__ __forceinline__ float* staged() { // two steps of eight parity boxes
+        extern __shared__ __align__(128) unsigned char march_smem[];
+        return reinterpret_cast<float*>(march_smem + ((128 - (smem_u32(march_smem) & 127)) & 127));
+    }
+    static __device__ __forceinline__ uint64_t* barriers() {
+        return reinterpret_cast<uint64_t*>(staged() + 2 * InvMarch::STAGE);
+    }
     template <bool Inside>
     static __device__ __forceinline__ void emit_step(const Out& out, f2 (&e)[8], f2 (&o)[8], int x, int y, int z,
                                                      bool live, int rows, int planes, int lane, f2& nonfinite);
@@ -163,9 +171,8 @@ __device__ __forceinline__ void InvMarchOp<Out>::run(const Params& P, uint32_t b
     using S = InvMarch;
     const InvLevel<float> lv = P.lv;
     const Out out = P.out;
-    extern __shared__ __align__(128) unsigned char march_smem[];
-    float* const stage = reinterpret_cast<float*>(march_smem + ((128 - (smem_u32(march_smem) & 127)) & 127));
-    uint64_t* const bar = reinterpret_cast<uint64_t*>(stage + 2 * S::STAGE);
+    float* const stage = staged();
+    uint64_t* const bar = barriers();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const Dims a = lv.a;
     const uint32_t strip = block % P.strips, zw = (block / P.strips) % P.zwins, sg = block / (P.strips * P.zwins);

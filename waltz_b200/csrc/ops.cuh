@@ -10,8 +10,12 @@
 //    body with its block index inside that entry (a chunk-tile work list).
 // Ops whose Params hold tensor maps use them in place: in kernel-parameter
 // space (grid constant) for op_kernel, in global memory for op_batch_kernel.
+// Such an op stages shared memory by tensor copies and declares
+//  * acquire_maps(params), before its maps in global memory are used;
+//  * kBarriers and barriers(), its copies' barriers in its shared memory.
 #pragma once
 #include "common.cuh"
+#include "tma.cuh"
 
 namespace wb {
 
@@ -80,7 +84,11 @@ __global__ void __launch_bounds__(Op::kThreads, Op::kMinBlocks)
 // pulling chunk-tile items (a field's block) from a device ticket until the
 // stage's items run out; an item runs the body exactly as op_batch_kernel
 // runs it, and the CTA synchronises before its next item reuses shared
-// memory. Items are taken in increasing order, so a stage whose blocks wait
+// memory. A staged op's next item writes the same buffers by tensor copies and
+// initialises the same barriers: every thread first orders its own accesses
+// before the copies' (they go through another proxy, which the block barrier
+// alone does not order), and thread 0, which initialises them again, ends the
+// barriers. Items are taken in increasing order, so a stage whose blocks wait
 // on earlier blocks of the same field (the WZP lookback) only waits on items
 // already running on resident CTAs. The ticket is zeroed before each launch.
 template <class Op>
@@ -105,7 +113,12 @@ __global__ void __launch_bounds__(Op::kThreads, Op::kMinBlocks)
             if (threadIdx.x == 0) Op::acquire_maps(table[lo]);
         }
         Op::run(table[lo], b - first, __ldg(starts + lo + 1) - first);
+        if constexpr (GridConstant<Op>::value) fence_proxy_async();
         __syncthreads(); // the item's shared memory and `item` are free again
+        if constexpr (GridConstant<Op>::value) {
+            if (threadIdx.x == 0)
+                for (int k = 0; k < Op::kBarriers; ++k) mbar_inval(Op::barriers() + k);
+        }
     }
 }
 

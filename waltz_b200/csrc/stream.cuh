@@ -86,6 +86,15 @@ template <class T, int UX, int UY, int Q, bool Z = true, int NT = 256> struct Fw
     static __device__ __forceinline__ void acquire_maps(const Params& P) {
         tensormap_acquire(&P.map);
     }
+    static constexpr int kBarriers = 1;
+    static __device__ __forceinline__ T* staged() { // [Q][FY][FX] input planes, [Q][UY][YP] after the Y pass
+        extern __shared__ __align__(128) unsigned char stream_smem[];
+        return reinterpret_cast<T*>(stream_smem + ((128 - (smem_u32(stream_smem) & 127)) & 127));
+    }
+    static __device__ __forceinline__ uint64_t* barriers() {
+        using S = StreamShape<T, UX, UY, Q, NT>;
+        return reinterpret_cast<uint64_t*>(staged() + S::IN + S::MID);
+    }
 };
 
 template <class T, int UX, int UY, int Q, bool Z, int NT>
@@ -99,10 +108,9 @@ __device__ __forceinline__ void FwdStreamOp<T, UX, UY, Q, Z, NT>::run(const Para
     using S = StreamShape<T, UX, UY, Q, NT>;
     using L = Lift<T>;
     using Bits = decltype(abs_bits(T(0)));
-    extern __shared__ __align__(128) unsigned char stream_smem[];
-    T* In = reinterpret_cast<T*>(stream_smem + ((128 - (smem_u32(stream_smem) & 127)) & 127)); // [Q][FY][FX]
-    T* Mid = In + S::IN;                                                                  // [Q][UY][YP]
-    uint64_t* bar = reinterpret_cast<uint64_t*>(Mid + S::MID);
+    T* In = staged();
+    T* Mid = In + S::IN;
+    uint64_t* bar = barriers();
     const int tid = threadIdx.x, warp = tid >> 5;
     const uint32_t bx = block % tiles_x, by = (block / tiles_x) % tiles_y;
     const uint32_t bzr = block / (tiles_x * tiles_y);
