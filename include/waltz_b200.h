@@ -228,6 +228,12 @@ int waltz_b200_wzp_encode_noalloc(const uint16_t* d_mag, const uint32_t* d_sign,
 int waltz_b200_test_lookback_timeout(const void* d_input, int width, uint32_t nx, uint32_t ny, uint32_t nz,
                                      double abs_error, void* d_archive, size_t capacity, uint32_t skip_chunk,
                                      uint32_t spin_cap, void* stream);
+/* Test hook for the bounded copy waits: waltz_b200_decompress with every copy
+ * wait of the staged float inverse levels giving up at its first poll (the
+ * copies then land while the kernels stop). Must fail with a copy-wait
+ * diagnostic on a float field that has such a level. */
+int waltz_b200_test_copy_timeout(const void* d_archive, size_t bytes, int width, uint32_t nx, uint32_t ny, uint32_t nz,
+                                 void* d_output, size_t output_bytes, void* stream);
 
 /* Instrumentation. waltz_b200_launch_count: kernels launched by this library
  * since load. waltz_b200_profile(1) makes the calling thread record CUDA

@@ -240,6 +240,24 @@ def test_lookback_wait_is_bounded():
     assert gpu_compress(a, 1e-3) == O.compress(a, 1e-3)
 
 
+@pytest.mark.parametrize("shape", [(64, 64, 64), (24, 24, 32)])
+def test_copy_wait_is_bounded(shape):
+    """Copy waits that run out stop the inverse march's blocks: the call fails
+    with a diagnostic, nothing hangs and the context stays usable."""
+    torch = _torch()
+    from waltz_b200 import synthetic as S
+    a = S.power_law_field(shape, 5)
+    archive = O.compress(a, 1e-3)
+    src = torch.from_numpy(np.frombuffer(archive, np.uint8).copy()).cuda()
+    out = torch.empty(shape, dtype=torch.float32, device="cuda")
+    nz, ny, nx = shape
+    rc = _lib().waltz_b200_test_copy_timeout(C.c_void_p(src.data_ptr()), len(archive), 4, nx, ny, nz,
+                                             C.c_void_p(out.data_ptr()), out.numel() * 4, _stream())
+    assert rc != 0
+    assert b"copy wait" in _lib().waltz_b200_last_error()
+    assert gpu_decompress(archive, shape, np.float32).tobytes() == O.decompress(archive, shape, np.float32).tobytes()
+
+
 def test_batch_decode_matches_oracle():
     """waltz_gpu_decode_batch: clipped edge tiles, two sides, a missing tile
     (fill), against per-tile oracle decodes."""

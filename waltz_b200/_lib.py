@@ -47,6 +47,8 @@ SIGNATURES = {
     "waltz_b200_test_lookback_timeout": (C.c_int, [C.c_void_p, C.c_int, C.c_uint32, C.c_uint32, C.c_uint32,
                                                    C.c_double, C.c_void_p, C.c_size_t, C.c_uint32, C.c_uint32,
                                                    C.c_void_p]),
+    "waltz_b200_test_copy_timeout": (C.c_int, [C.c_void_p, C.c_size_t, C.c_int, C.c_uint32, C.c_uint32, C.c_uint32,
+                                               C.c_void_p, C.c_size_t, C.c_void_p]),
     "waltz_b200_launch_count": (C.c_ulonglong, []),
     "waltz_b200_graph_count": (C.c_ulonglong, []),
     "waltz_b200_profile": (None, [C.c_int]),

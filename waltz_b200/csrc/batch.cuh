@@ -123,6 +123,7 @@ static void decode_batch(const waltz_batch_shape& d, const uint8_t* host, const 
     uint32_t word = 0;
     check(cudaMemcpyAsync(&word, status, 4, cudaMemcpyDeviceToHost, stream), "readback");
     check(cudaStreamSynchronize(stream), "batch decode");
+    if (word & ST_WAIT_TIMEOUT) throw Error("Waltz: asynchronous copy wait exceeded its bound");
     if (word & ST_DIRECTORY) {
         // Non-canonical group order: exact check on the host copy.
         for (const Job& job : list)
@@ -137,7 +138,6 @@ static void decode_batch(const waltz_batch_shape& d, const uint8_t* host, const 
     if (word & ST_BAD_QOUT) throw Error("invalid quantization outlier");
     if (word & ST_BAD_REPAIR) throw Error("nonfinite correction");
     if (word & ST_NONFINITE_INPUT) throw Error("nonfinite reconstruction");
-    if (word & ST_WAIT_TIMEOUT) throw Error("Waltz: asynchronous copy wait exceeded its bound");
 }
 
 } // namespace wb

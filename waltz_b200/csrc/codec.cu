@@ -201,6 +201,8 @@ struct Options {
     uint64_t small_march_fwd = 0; // dyadic forward levels of at most this many samples: XY march + Z march
 };
 static thread_local Options t_opt;
+// Polls of the float inverse levels' copy waits (a test hook lowers it).
+static thread_local uint32_t t_copy_polls = kWaitBound;
 
 // One Z level of the plane schedule as a per-column register march
 // (ZMarchOp): a warp per 32 columns and run of windows. A single field's
@@ -377,6 +379,7 @@ static bool level_inv(const InvSrc<float>& src, Dims a, const Out& out, uint32_t
     p.lv = InvLevel<float>{src.base, src.sy, src.sz, src.low, src.lo, a};
     p.out = out;
     p.status = status;
+    p.wait_bound = t_copy_polls;
     sink.run<Op>(p, uint32_t(blocks), S::smem);
     return true;
 }
@@ -1314,12 +1317,13 @@ template <class T> struct CompressJob {
     size_t finish(const uint64_t* h) const {
         const uint32_t status = uint32_t(h[8]);
         const uint64_t np = h[5], nq = h[6];
+        // first: what the stages after a copy that never landed report follows from it
+        if (status & ST_WAIT_TIMEOUT) throw Error("Waltz: asynchronous copy wait exceeded its bound");
         if (status & ST_NONFINITE_INPUT) throw Error("nonfinite input is unsupported");
         if (status & ST_MATRIX_RANGE) throw Error("Waltz: the matrix form needs samples within the float range");
         if (status & ST_QUANT_DOMAIN) throw Error("coefficient exceeds portable integer conversion domain");
         if (status & ST_BOUND) throw Error("native repair cannot meet strict bound or nonfinite reconstruction");
         if (status & ST_LOOKBACK_TIMEOUT) throw Error("Waltz: WZP lookback wait exceeded its bound");
-        if (status & ST_WAIT_TIMEOUT) throw Error("Waltz: asynchronous copy wait exceeded its bound");
         if (status & ST_CAPACITY) throw Error("archive capacity too small");
         if ((n > (1u << 20) && nq >= (1u << 20)) || (n > (1u << 22) && np >= (1u << 22)))
             throw Error("portable GPU side-channel capacity reached");
@@ -1499,6 +1503,8 @@ static void decode_finish(uint32_t status, const uint8_t* d_in, const Header& h,
                           uint32_t* d_status, uint32_t* seen, cudaStream_t stream) {
     uint64_t* pin = pinned();
     const uint64_t header = wzp_header(uint32_t(g.n));
+    // first: what the stages after a copy that never landed report follows from it
+    if (status & ST_WAIT_TIMEOUT) throw Error("Waltz: asynchronous copy wait exceeded its bound");
     if (status & ST_DIRECTORY) {
         std::vector<uint8_t> dir(header);
         check(cudaMemcpy(dir.data(), d_in + 32, header, cudaMemcpyDeviceToHost), "directory readback");
@@ -1524,7 +1530,6 @@ static void decode_finish(uint32_t status, const uint8_t* d_in, const Header& h,
     if (status & ST_BAD_QOUT) throw Error("invalid quantization outlier");
     if (status & ST_BAD_REPAIR) throw Error("nonfinite correction");
     if (status & ST_NONFINITE_INPUT) throw Error("nonfinite reconstruction");
-    if (status & ST_WAIT_TIMEOUT) throw Error("Waltz: asynchronous copy wait exceeded its bound");
 }
 
 template <class T>
@@ -2514,6 +2519,15 @@ extern "C" int waltz_b200_test_lookback_timeout(const void* d_input, int width, 
     } catch (const std::exception& e) {
         return fail(e);
     }
+}
+
+// Test hook: decode with the float inverse levels' copy waits giving up at once.
+extern "C" int waltz_b200_test_copy_timeout(const void* d_archive, size_t bytes, int width, uint32_t nx, uint32_t ny,
+                                            uint32_t nz, void* d_output, size_t output_bytes, void* stream) {
+    t_copy_polls = 0;
+    const int rc = waltz_b200_decompress(d_archive, bytes, width, nx, ny, nz, d_output, output_bytes, stream);
+    t_copy_polls = kWaitBound;
+    return rc;
 }
 
 #include "batch.cuh"

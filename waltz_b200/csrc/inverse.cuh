@@ -65,7 +65,7 @@ template <class T, int UX, int UY, int UZ, class Out> struct InvTileOp {
         Out out;
         uint32_t* status;
     };
-    static __device__ __forceinline__ void run(const Params& P, uint32_t block, uint32_t);
+    static __device__ __forceinline__ bool run(const Params& P, uint32_t block, uint32_t);
     static __device__ __forceinline__ void acquire_maps(const Params& P) {
         tensormap_acquire(&P.cmap);
         if (P.lv.low) tensormap_acquire(&P.lmap);
@@ -81,7 +81,7 @@ template <class T, int UX, int UY, int UZ, class Out> struct InvTileOp {
 };
 
 template <class T, int UX, int UY, int UZ, class Out>
-__device__ __forceinline__ void InvTileOp<T, UX, UY, UZ, Out>::run(const Params& P, uint32_t block, uint32_t) {
+__device__ __forceinline__ bool InvTileOp<T, UX, UY, UZ, Out>::run(const Params& P, uint32_t block, uint32_t) {
     const InvLevel<T> lv = P.lv;
     const uint32_t tiles_x = P.tiles_x, tiles_y = P.tiles_y;
     const Out out = P.out;
@@ -141,11 +141,11 @@ __device__ __forceinline__ void InvTileOp<T, UX, UY, UZ, Out>::run(const Params&
             bool landed = true;
             if (warp == 0) {
 #pragma unroll 1
-                for (int p = 0; p < 4; ++p) landed = landed && mbar_wait(bar + p, 0, kWaitBound);
+                for (int p = 0; p < 4; ++p) landed = mbar_wait(bar + p, 0, kWaitBound) && landed;
             }
             if (!__syncthreads_and(landed)) {
                 if (tid == 0) atomicOr(status, ST_WAIT_TIMEOUT);
-                return;
+                return false;
             }
         }
         // only the cells outside the array: the in-range footprint is the box
@@ -202,9 +202,9 @@ __device__ __forceinline__ void InvTileOp<T, UX, UY, UZ, Out>::run(const Params&
     // Pair j of a line sits at slot j of the z-even and z-odd boxes, and the
     // outputs of pair j overwrite exactly those two slots.
     constexpr int ZS = S::HY * S::BX; // z-slot stride inside a box
+    bool failed = false; // a copy that never landed: skip the work, the status fails the call
     {
         constexpr int P = UZ / 2 + 4;
-        bool failed = false; // a copy that never landed: skip the work, the status fails the call
         for (int L = tid; L < S::FX * S::FY; L += kThreads) {
             // x index fastest inside one (x parity, y parity) box
             const int i = L % (S::FX / 2), k = (L / (S::FX / 2)) % (S::FY / 2);
@@ -321,6 +321,7 @@ __device__ __forceinline__ void InvTileOp<T, UX, UY, UZ, Out>::run(const Params&
             }
         }
     }
+    return !failed;
 }
 
 // ---------------------------------------------------------------------------
@@ -361,7 +362,7 @@ template <class T, int UX, int UY, int UZ, class Out> struct InvTileXYOp {
         Out out;
         uint32_t* status;
     };
-    static __device__ __forceinline__ void run(const Params& P, uint32_t block, uint32_t);
+    static __device__ __forceinline__ bool run(const Params& P, uint32_t block, uint32_t);
     static __device__ __forceinline__ void acquire_maps(const Params& P) {
         tensormap_acquire(&P.cmap);
         if (P.lv.low) tensormap_acquire(&P.lmap);
@@ -377,7 +378,7 @@ template <class T, int UX, int UY, int UZ, class Out> struct InvTileXYOp {
 };
 
 template <class T, int UX, int UY, int UZ, class Out>
-__device__ __forceinline__ void InvTileXYOp<T, UX, UY, UZ, Out>::run(const Params& P, uint32_t block, uint32_t) {
+__device__ __forceinline__ bool InvTileXYOp<T, UX, UY, UZ, Out>::run(const Params& P, uint32_t block, uint32_t) {
     const InvLevel<T> lv = P.lv;
     const uint32_t tiles_x = P.tiles_x, tiles_y = P.tiles_y;
     const Out out = P.out;
@@ -416,7 +417,7 @@ __device__ __forceinline__ void InvTileXYOp<T, UX, UY, UZ, Out>::run(const Param
         const bool ok = __syncthreads_and(warp != 0 || mbar_wait(bar, 0, kWaitBound));
         if (!ok) {
             if (tid == 0) atomicOr(status, ST_WAIT_TIMEOUT);
-            return;
+            return false;
         }
     }
     // ---- edge tiles: out-of-range cells of the in-array planes from their
@@ -542,6 +543,7 @@ __device__ __forceinline__ void InvTileXYOp<T, UX, UY, UZ, Out>::run(const Param
             }
         }
     }
+    return true;
 }
 
 } // namespace wb

@@ -82,8 +82,9 @@ template <class Out> struct InvMarchOp {
         uint32_t seg;           // Y windows per CTA
         Out out;
         uint32_t* status;
+        uint32_t wait_bound;    // polls of a copy wait
     };
-    static __device__ __forceinline__ void run(const Params& P, uint32_t block, uint32_t);
+    static __device__ __forceinline__ bool run(const Params& P, uint32_t block, uint32_t);
     static __device__ __forceinline__ void acquire_maps(const Params& P) {
         tensormap_acquire(&P.cmap);
         if (P.lv.low) tensormap_acquire(&P.lmap);
@@ -167,7 +168,7 @@ __device__ __forceinline__ void InvMarchOp<Out>::emit_step(const Out& out, f2 (&
 }
 
 template <class Out>
-__device__ __forceinline__ void InvMarchOp<Out>::run(const Params& P, uint32_t block, uint32_t) {
+__device__ __forceinline__ bool InvMarchOp<Out>::run(const Params& P, uint32_t block, uint32_t) {
     using S = InvMarch;
     const InvLevel<float> lv = P.lv;
     const Out out = P.out;
@@ -227,7 +228,6 @@ __device__ __forceinline__ void InvMarchOp<Out>::run(const Params& P, uint32_t b
     __syncthreads();
 
     f2 ke[4], ko[4]; // the Y pass's kept row pairs (lifted along Z and X)
-    bool failed = false;
     f2 nonfinite = 0; // interior samples times zero, summed: NaN once one was not finite
 #pragma unroll 1
     for (int t = 0; t <= nw; ++t) {
@@ -241,12 +241,7 @@ __device__ __forceinline__ void InvMarchOp<Out>::run(const Params& P, uint32_t b
                 if (gy < a.y && gz < a.z) out.warm(min(uint32_t(ox + S::SHIFT), a.x - 1), gy, gz); // most of the row
             }
         }
-        // a copy that never lands: the status fails the call, and the later
-        // steps go on without waiting
-        if (!failed && !mbar_wait(bar + (t & 1), uint32_t(t >> 1) & 1u, kWaitBound)) {
-            failed = true;
-            atomicOr(P.status, ST_WAIT_TIMEOUT);
-        }
+        const bool landed = mbar_wait(bar + (t & 1), uint32_t(t >> 1) & 1u, P.wait_bound);
         // ---- rows outside the level, from their reflections (coefficient
         // mapped): copied from the staged rows when the reflected row is among
         // them, else loaded; cells inside the level along x and z only
@@ -308,7 +303,17 @@ __device__ __forceinline__ void InvMarchOp<Out>::run(const Params& P, uint32_t b
             }
         }
         fence_proxy_async(); // this thread's accesses to the other buffer precede the copies into it
-        __syncthreads();
+        if (!__syncthreads_and(landed)) {
+            // a copy that did not land: the block stops as a whole, with no
+            // further copy issued. Those in flight (this step's, and at the
+            // start the next one's) get as long again to end.
+            if (tid == 0) {
+                atomicOr(P.status, ST_WAIT_TIMEOUT);
+                mbar_wait(bar + (t & 1), uint32_t(t >> 1) & 1u, kWaitBound);
+                if (t == 0) mbar_wait(bar + 1, 0, kWaitBound);
+            }
+            return false;
+        }
         // every thread has left the previous step: its buffer takes the next one
         if (tid == 0 && t > 0 && t < nw) issue(t + 1);
         if (edge_x) { // both sides of one Z output row per thread pair
@@ -381,6 +386,7 @@ __device__ __forceinline__ void InvMarchOp<Out>::run(const Params& P, uint32_t b
         if (d.status && __any_sync(0xffffffffu, !(n0 == 0.f && n1 == 0.f)) && lane == 0)
             atomicOr(d.status, ST_NONFINITE_INPUT);
     }
+    return true;
 }
 
 } // namespace wb

@@ -12,7 +12,8 @@
 // space (grid constant) for op_kernel, in global memory for op_batch_kernel.
 // Such an op stages shared memory by tensor copies and declares
 //  * acquire_maps(params), before its maps in global memory are used;
-//  * kBarriers and barriers(), its copies' barriers in its shared memory.
+//  * kBarriers and barriers(), its copies' barriers in its shared memory;
+// its run() returns whether every copy this thread waited for landed.
 #pragma once
 #include "common.cuh"
 #include "tma.cuh"
@@ -112,12 +113,17 @@ __global__ void __launch_bounds__(Op::kThreads, Op::kMinBlocks)
         if constexpr (GridConstant<Op>::value) {
             if (threadIdx.x == 0) Op::acquire_maps(table[lo]);
         }
-        Op::run(table[lo], b - first, __ldg(starts + lo + 1) - first);
-        if constexpr (GridConstant<Op>::value) fence_proxy_async();
-        __syncthreads(); // the item's shared memory and `item` are free again
         if constexpr (GridConstant<Op>::value) {
+            const bool landed = Op::run(table[lo], b - first, __ldg(starts + lo + 1) - first);
+            fence_proxy_async();
+            // a copy that did not land may still come: this CTA takes no
+            // further item (the item's status fails the call)
+            if (!__syncthreads_and(landed)) return;
             if (threadIdx.x == 0)
                 for (int k = 0; k < Op::kBarriers; ++k) mbar_inval(Op::barriers() + k);
+        } else {
+            Op::run(table[lo], b - first, __ldg(starts + lo + 1) - first);
+            __syncthreads(); // the item's shared memory and `item` are free again
         }
     }
 }

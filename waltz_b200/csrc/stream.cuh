@@ -82,7 +82,7 @@ template <class T, int UX, int UY, int Q, bool Z = true, int NT = 256> struct Fw
         FwdOut<T> out;
         uint32_t* status;
     };
-    static __device__ __forceinline__ void run(const Params& P, uint32_t block, uint32_t);
+    static __device__ __forceinline__ bool run(const Params& P, uint32_t block, uint32_t);
     static __device__ __forceinline__ void acquire_maps(const Params& P) {
         tensormap_acquire(&P.map);
     }
@@ -98,7 +98,7 @@ template <class T, int UX, int UY, int Q, bool Z = true, int NT = 256> struct Fw
 };
 
 template <class T, int UX, int UY, int Q, bool Z, int NT>
-__device__ __forceinline__ void FwdStreamOp<T, UX, UY, Q, Z, NT>::run(const Params& P, uint32_t block, uint32_t) {
+__device__ __forceinline__ bool FwdStreamOp<T, UX, UY, Q, Z, NT>::run(const Params& P, uint32_t block, uint32_t) {
     const FwdSrc<T> src = P.src;
     const Dims a = P.a;
     const uint32_t tiles_x = P.tiles_x, tiles_y = P.tiles_y, zrange = P.zrange;
@@ -116,7 +116,6 @@ __device__ __forceinline__ void FwdStreamOp<T, UX, UY, Q, Z, NT>::run(const Para
     const uint32_t bzr = block / (tiles_x * tiles_y);
     const uint32_t ox = bx * UX, oy = by * UY;
     const uint32_t z0 = bzr * zrange, z1 = min(a.z, z0 + zrange);
-    if (z0 >= z1) return;
     // input planes [zin0, zin1): with Z, pairs from z0 - 4 until the pair
     // that completes output z1 - 1; an XY level reads its output planes only
     const int64_t zin0 = Z ? int64_t(z0) - 4 : int64_t(z0);
@@ -168,7 +167,7 @@ __device__ __forceinline__ void FwdStreamOp<T, UX, UY, Q, Z, NT>::run(const Para
             const bool ok = __syncthreads_and(warp != 0 || mbar_wait(bar, phase, kWaitBound));
             if (!ok) {
                 if (tid == 0) atomicOr(status, ST_WAIT_TIMEOUT);
-                return;
+                return false;
             }
             phase ^= 1;
             if (edge) {
@@ -319,6 +318,7 @@ __device__ __forceinline__ void FwdStreamOp<T, UX, UY, Q, Z, NT>::run(const Para
     if (check) {
         if (__syncthreads_or(nonfinite_max(seen)) && threadIdx.x == 0) atomicOr(src.status, ST_NONFINITE_INPUT);
     }
+    return true;
 }
 
 } // namespace wb

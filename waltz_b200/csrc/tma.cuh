@@ -3,9 +3,9 @@
 //
 // Device side: one elected thread arms the barrier with the expected byte
 // count and issues the copies; every thread waits on the barrier's phase with
-// an iteration bound, after which the block agrees (barrier vote) to stop and
-// records ST_WAIT_TIMEOUT instead of hanging. Copies are plain, one CTA
-// each: every CTA reads its own boxes into its own shared memory.
+// an iteration bound, after which the block stops and records ST_WAIT_TIMEOUT
+// instead of hanging. Copies are plain, one CTA each: every CTA reads its own
+// boxes into its own shared memory.
 // Host side: tensor maps are encoded with the driver's cuTensorMapEncodeTiled,
 // reached through the runtime's driver entry point (no link-time libcuda).
 #pragma once
@@ -66,10 +66,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
 }
 
 // Poll bound of every wait for a TMA copy or an MMA. A CTA whose wait runs
-// out records ST_WAIT_TIMEOUT and returns, and the host rejects the call. The
-// bulk copy it waited on may still be in flight into the CTA's shared memory
-// at that point. A healthy device lands a tile in microseconds, far inside
-// 2^22 polls, so this path only runs on a device that has already failed.
+// out records ST_WAIT_TIMEOUT, issues no further copy and returns, and the
+// host rejects the call. (The float inverse march gives its copies in flight
+// the same bound again first.) The bulk copy it waited on may still be in
+// flight into the CTA's shared memory at that point. A healthy device lands a
+// tile in microseconds, far inside 2^22 polls, so this path only runs on a
+// device that has already failed.
 constexpr uint32_t kWaitBound = 1u << 22;
 
 // A tensor map read from global memory (a batched launch's parameter table)
