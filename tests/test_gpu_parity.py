@@ -477,6 +477,32 @@ def test_work_queue_items_reuse_the_staged_buffers(dtype, shape):
         lib.waltz_b200_batch_config(1, 32)
 
 
+def test_batch_results_are_written_in_place_like_slices():
+    """The tensors of a batch decode take in-place operations that autograd
+    records, with and without a caller's buffer (here one that does not start
+    at its storage's beginning); the archives of a batch compress too."""
+    torch = _torch()
+    import waltz_b200
+    fields, bounds = _uneven_batch(torch, 12, 3)
+    shapes = [tuple(f.shape) for f in fields]
+    room = sum(f.numel() for f in fields)
+    archives = waltz_b200.compress_batch(fields, bounds)
+    w = torch.full((1,), 2.0, device="cuda", requires_grad=True)
+    for out in (None, torch.empty(room + 5, device="cuda")[5:]):
+        views = waltz_b200.decompress_batch(archives, shapes, torch.float32, out=out)
+        expect = [waltz_b200.decompress_tensor(a, s, torch.float32) for a, s in zip(archives, shapes)]
+        assert all(torch.equal(v, e) for v, e in zip(views, expect))
+        if out is not None:
+            assert views[1].data_ptr() == out.data_ptr() + 4 * fields[0].numel()
+        views[1].mul_(w)
+        views[1].square().sum().backward()  # d/dw of sum (v w)^2
+        assert torch.allclose(w.grad.double(), 2 * 2 * expect[1].double().square().sum(), rtol=1e-3)
+        assert torch.equal(views[0], expect[0]) and torch.equal(views[2], expect[2])
+        w.grad = None
+    archives[0].copy_(torch.ones(archives[0].numel(), device="cuda", requires_grad=True))
+    assert bool((archives[0] == 1).all())
+
+
 def _uneven_batch(torch, seed, count, sides=(16, 17, 32, 48, 64)):
     from waltz_b200 import synthetic as S
     rng = np.random.default_rng(seed)

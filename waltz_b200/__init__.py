@@ -73,6 +73,17 @@ def _fill_dims(items, shapes, itemsize):
         items[name] = dims[:, k]
 
 
+def _view(out, shape, at):
+    """A dense view of `shape` at element `at` of out's storage, in one call. It
+    may be written in place like a slice; the views of one split() may not,
+    once autograd records the write."""
+    strides, step = [], 1
+    for n in reversed(shape):
+        strides.append(step)
+        step *= n
+    return out.as_strided(shape, strides[::-1], at)
+
+
 def _stream(torch, stream):
     s = stream if stream is not None else torch.cuda.current_stream()
     return C.c_void_p(s.cuda_stream)
@@ -191,12 +202,8 @@ def compress_batch(fields, abs_errors, *, out=None, stream=None, tuned=True):
         autotune.apply_batch(lib(), shapes, itemsize)
     checked(lib().waltz_b200_compress_batch((Chunk * len(fields)).from_buffer(items), len(fields), itemsize, written,
                                             _stream(torch, stream)))
-    # the archives and the gaps between them, in one call
-    pieces, at = [], 0
-    for off, size in zip(offsets, written):
-        pieces += (off - at, size)
-        at = off + size
-    return list(out[:at].split(pieces)[1::2])
+    base = out.storage_offset()
+    return [_view(out, (size,), base + off) for off, size in zip(offsets, written)]
 
 
 def decompress_batch(archives, shapes, dtype, *, out=None, headers=None, stream=None, tuned=True):
@@ -232,7 +239,10 @@ def decompress_batch(archives, shapes, dtype, *, out=None, headers=None, stream=
     else:
         if out.dtype != dtype or not out.is_contiguous() or out.numel() < sum(sizes):
             raise ValueError(f"out must be a contiguous {dtype} tensor of at least {sum(sizes)} samples")
-        views = [v.view(s) for v, s in zip(out.view(-1)[:sum(sizes)].split(sizes), shapes)]
+        views, at = [], out.storage_offset()
+        for s, size in zip(shapes, sizes):
+            views.append(_view(out, s, at))
+            at += size
     items = np.zeros(len(archives), _ARCHIVE)
     items["archive"] = [a.data_ptr() for a in archives]
     items["bytes"] = [a.numel() for a in archives]
