@@ -96,3 +96,11 @@ def test_noalloc_encoder_host_checks_without_a_device():
         assert message in _lib.last_error()
         if dm is not None:
             assert written.value == 0
+
+
+def test_capacity_refuses_what_it_refuses_whatever_came_before():
+    import waltz_b200
+    assert waltz_b200.compressed_capacity(4096, 4) > 4096 * 2
+    for n in (4096.0, "4096"):
+        with pytest.raises(ctypes.ArgumentError):
+            waltz_b200.compressed_capacity(n, 4)

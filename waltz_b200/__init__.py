@@ -53,9 +53,13 @@ def _bound(value):
     return value
 
 
-@lru_cache(maxsize=4096)
 def compressed_capacity(n: int, itemsize: int) -> int:
     return int(lib().waltz_b200_compressed_capacity(n, itemsize))
+
+
+# The same for the sample counts of the batch calls' own shapes. (The public
+# call takes any argument, and 4096.0 finds the entry of 4096.)
+_capacity = lru_cache(maxsize=4096)(compressed_capacity)
 
 
 # The batch calls' item structures (Chunk, Archive), filled a column at a time.
@@ -181,7 +185,7 @@ def compress_batch(fields, abs_errors, *, out=None, stream=None, tuned=True):
     if len(bounds) != len(fields):
         raise ValueError("one bound per field")
     shapes = [tuple(f.shape) for f in fields]
-    caps = [compressed_capacity(math.prod(shape), itemsize) for shape in shapes]
+    caps = [_capacity(math.prod(shape), itemsize) for shape in shapes]
     offsets, total = [], 0
     for cap in caps:
         total = (total + 15) // 16 * 16
