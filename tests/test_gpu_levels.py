@@ -65,3 +65,33 @@ def test_matrix_repairs_with_a_partial_last_warp(form, dtype):
     assert np.abs(out.astype(np.float64) - a.astype(np.float64)).max() <= eb
     assert waltz_b200.decompress(archive, shape=a.shape, dtype=dtype).tobytes() == out.tobytes()
     assert waltz_b200.compress(a, abs_error=eb, form=form) == archive
+
+
+_ROUND_TRIP = """
+import ctypes as C, sys, torch
+from waltz_b200 import _lib
+z, y, x = 1040, 2048, 2056
+assert z * y * x > 1 << 32
+a = torch.empty((z, y, x), device="cuda").normal_(generator=torch.Generator("cuda").manual_seed(3))
+b = a.clone()
+for inverse in (0, 1):
+    _lib.checked(_lib.lib().waltz_b200_transform(C.c_void_p(b.data_ptr()), 4, x, y, z, inverse,
+                                                 C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+worst = max(float((p - q).abs().max()) for p, q in zip(a.split(40), b.split(40)))
+print("worst", worst)
+sys.exit(worst > 1e-3)
+"""
+
+
+def test_transform_of_more_than_2_to_the_32_samples():
+    """The transform entry takes any size: forward and inverse of 4.4e9 samples
+    give the field back (rounding alone: about 1e-5 of samples of order one).
+    In a process of its own, whose scratch ends with it."""
+    import subprocess
+    import sys
+
+    import torch
+    if torch.cuda.mem_get_info()[0] < 110 << 30:
+        pytest.skip("needs 110 GiB of device memory")
+    r = subprocess.run([sys.executable, "-c", _ROUND_TRIP], capture_output=True, text=True, timeout=240)
+    assert r.returncode == 0, r.stdout + r.stderr

@@ -263,13 +263,15 @@ template <class K> static uint64_t resident_slots(K kernel, size_t smem, int thr
 // ranges only as far as needed to give every resident CTA slot work (one
 // range per column tile when many fields share the GPU). Planes are staged by
 // TMA; returns false, with nothing launched, when the source rows do not meet
-// the copy engine's alignment.
+// the copy engine's alignment or an output offset of the level needs more
+// than the kernel's 32 bits (the transform entry alone takes such fields).
 template <class T, bool Z, int NT>
 static bool level_fwd_stream_nt(const FwdSrc<T>& src, Dims a, const FwdOut<T>& out, uint32_t* status, Sink& sink) {
     constexpr int UX = StreamTile<T>::UX, UY = StreamTile<T>::UY, Q = StreamTile<T>::Q;
     using S = StreamShape<T, UX, UY, Q, NT>;
     using Op = FwdStreamOp<T, UX, UY, Q, Z, NT>;
     typename Op::Params p{};
+    if (uint64_t(a.z) * out.sz > 0xffffffffull) return false;
     if (!make_map_3d<T>(&p.map, src.p, a.x, a.y, a.z, src.sy, src.sz, S::FX, S::FY, 1)) return false;
     const uint32_t tx = (a.x + UX - 1) / UX, ty = (a.y + UY - 1) / UY;
     const uint64_t tiles = uint64_t(tx) * ty;

@@ -125,8 +125,8 @@ __device__ __forceinline__ bool FwdStreamOp<T, UX, UY, Q, Z, NT>::run(const Para
     const int fx_lo = ox < 4 ? int(4 - ox) : 0, fx_hi = min(S::FX, int(a.x - ox) + 4);
     const int fy_lo = oy < 4 ? int(4 - oy) : 0, fy_hi = min(S::FY, int(a.y - oy) + 4);
 
-    // per-thread output columns: x/y parts of the split addresses, 32 bits (a
-    // field has fewer than 2^32 samples): with 64 the 256-thread float kernel
+    // per-thread output columns: x/y parts of the split addresses, 32 bits (the
+    // launcher keeps larger levels out): with 64 the 256-thread float kernel
     // spilled at its 64 registers (512^3 finest level 0.425 -> 0.367 ms)
     uint32_t hi_off[S::CPT], lo_off[S::CPT];
     bool even_xy[S::CPT];
