@@ -75,3 +75,21 @@ def test_matrix_choice_lookup(tmp_path):
     assert A.matrix_choice((64, 1024, 1024), 4, path) == "matrix-bf16"
     assert A.matrix_choice((96, 256, 384), 8, path) is None
     assert A.matrix_choice((512, 512, 512), 4, path) is None  # dyadic: no entry of that schedule
+
+
+def test_candidates_differ_in_acting_knobs_only():
+    full = [{**c, "small_march": sm, "small_march_fwd": mf} for sm in A.SMALL_MARCH_CHOICES
+            for mf in A.SMALL_MARCH_FWD_CHOICES for c in A.SINGLE_CANDIDATES]
+    f32 = A.candidates(full, "f32", "dyadic")
+    f64 = A.candidates(full, "f64", "dyadic")
+    assert all(set(c) == {"zmarch", "small_fwd"} for c in f32) and len(f32) == 2 * 4
+    assert all(set(c) == {"zmarch", "small_fwd", "small_inv"} for c in f64)
+    assert {c["small_inv"] for c in f64} == {1 << 15, 1 << 18, 1 << 21, 1 << 24, 1 << 27}
+    plane = A.candidates(A.SINGLE_CANDIDATES, "f32", "plane")
+    assert all("zmarch" not in c and "small_march" not in c for c in plane) and len(plane) == 2 * 3 * 4
+    batch = A.candidates(A.BATCH_CANDIDATES, "f32")
+    assert all("small_march" not in c for c in batch) and len(batch) < len(A.BATCH_CANDIDATES)
+    assert any(c.get("small_march") for c in A.candidates(A.BATCH_CANDIDATES, "f64"))
+    # a reduced candidate sets what the full one set, as far as it acts
+    for c in full:
+        assert A.acting(A.acting(c, "f64", "dyadic"), "f64", "dyadic") == A.acting(c, "f64", "dyadic")

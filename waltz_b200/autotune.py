@@ -21,7 +21,9 @@ question and the table can be applied blindly):
    and an XY march instead of the tile inverse (WALTZ_B200_OPT_SMALL_MARCH;
    float levels take the y-march at every size), and
    dyadic forward levels as an XY march and a Z march instead of the
-   z-march (WALTZ_B200_OPT_SMALL_MARCH_FWD); single dyadic fields try both;
+   z-march (WALTZ_B200_OPT_SMALL_MARCH_FWD); single dyadic fields try both.
+   Of a class's candidates only those that differ in a knob acting on it are
+   timed (acting());
  * the transform form (lifting or one split of the tensor-core matrix form)
    of fields the matrix form serves: every split is timed and the fastest
    one that beats lifting by 3 % with a compression ratio at most 2 % lower
@@ -52,7 +54,7 @@ OPT_SMALL_MARCH, OPT_SMALL_MARCH_FWD = 7, 8
 BATCH_STAGES, BATCH_FIELDS, BATCH_QUEUE = 0, 1, 2
 DEFAULT_SINGLE = {"stage_kernels": 1, "zmarch": 0, "small_inv": 1 << 15, "small_fwd": 1 << 20, "xy_march": 0,
                   "small_march": 0, "small_march_fwd": 0}
-SMALL_MARCH_CHOICES = (0, 1 << 21, 1 << 24, 1 << 27)  # dyadic inverse levels as Z + XY marches up to this size
+SMALL_MARCH_CHOICES = (0, 1 << 21, 1 << 24, 1 << 27)  # double dyadic inverse levels as marches up to this size
 SMALL_MARCH_FWD_CHOICES = (0, 1 << 21, 1 << 24)       # the same for dyadic forward levels
 MATRIX_MARGIN = 0.97  # the matrix form changes the header flag: take it only for a clear gain
 MATRIX_RATIO = 0.98   # ... and only when its archive stays within 2 % of the plain one's size
@@ -93,6 +95,35 @@ BATCH_CANDIDATES = ([{"mode": BATCH_STAGES, "width": w, "stage_kernels": s, "zma
                      for w in (4, 16) for s in (1, 0) for z in (0, 32) for xy in (0, 3) for mf in (0, 1 << 24)] +
                     [{"mode": BATCH_QUEUE, "width": w, "stage_kernels": s} for w in (1, 4, 16) for s in (1, 0)] +
                     [{"mode": BATCH_FIELDS, "width": w, "stage_kernels": s} for w in (16, 32, 64) for s in (1, 0)])
+
+
+def acting(knobs, dtype, schedule=None):
+    """The knobs of a candidate that act on fields of this type and schedule
+    (None: a batch, which holds both): candidates equal in these are one.
+     * dyadic fields run no plane stage; their forward levels march up to the
+       larger of small_fwd and small_march_fwd, their inverse levels, of
+       doubles only, up to the larger of small_inv and small_march (float ones
+       are staged at every size);
+     * plane fields have no dyadic z-march and no dyadic levels;
+     * a batch of floats has no inverse level that small_march acts on."""
+    k = {**DEFAULT_SINGLE, **knobs}
+    if schedule == "dyadic":
+        a = {"zmarch": k["zmarch"], "small_fwd": max(k["small_fwd"], k["small_march_fwd"])}
+        if dtype == "f64":
+            a["small_inv"] = max(k["small_inv"], k["small_march"])
+        return a
+    if schedule == "plane":
+        return {n: k[n] for n in ("stage_kernels", "small_inv", "small_fwd", "xy_march")}
+    return {n: v for n, v in knobs.items() if n != "small_march" or dtype == "f64"}
+
+
+def candidates(cands, dtype, schedule=None):
+    """The distinct candidates of a list, each reduced to its acting knobs."""
+    unique = {}
+    for c in cands:
+        a = acting(c, dtype, schedule)
+        unique.setdefault(tuple(sorted(({**DEFAULT_SINGLE, **a} if schedule is None else a).items())), a)
+    return list(unique.values())
 
 
 def _levels(n):
@@ -208,21 +239,21 @@ def _tune_single(torch, lib, shape, dtype, reps, rel=1e-3):
     eb = rel * (hi - lo)
     itemsize = f.element_size()
     results = []
-    # plane fields also try their XY levels as the warp march
-    cands = SINGLE_CANDIDATES
-    if single_class(shape, itemsize)["schedule"] == "plane":
-        cands = cands + [{**c, "xy_march": xy} for xy in (1, 2, 3) for c in SINGLE_CANDIDATES]
+    cls = single_class(shape, itemsize)
+    # plane fields also try their XY levels as the warp march, dyadic ones
+    # their levels as marches up to other sizes
+    if cls["schedule"] == "plane":
+        cands = SINGLE_CANDIDATES + [{**c, "xy_march": xy} for xy in (1, 2, 3) for c in SINGLE_CANDIDATES]
     else:
-        # dyadic fields also try their small inverse levels as marches
         cands = [{**c, "small_march": sm, "small_march_fwd": mf} for sm in SMALL_MARCH_CHOICES
                  for mf in SMALL_MARCH_FWD_CHOICES for c in SINGLE_CANDIDATES]
-    for cand in cands:
+    for cand in candidates(cands, cls["dtype"], cls["schedule"]):
         set_single(lib, cand)
         arc = waltz_b200.compress_tensor(f, eb, tuned=False)
         tc = _time(torch, lambda: waltz_b200.compress_tensor(f, eb, tuned=False), reps)
         td = _time(torch, lambda: waltz_b200.decompress_tensor(arc, shape, dtype, tuned=False), reps)
         results.append({"knobs": cand, "compress_ms": round(tc, 4), "decompress_ms": round(td, 4)})
-    entry = {"class": single_class(shape, itemsize), "workload": f"{dtype} {shape} k^-11/3 REL {rel:g}",
+    entry = {"class": cls, "workload": f"{dtype} {shape} k^-11/3 REL {rel:g}",
              "measured": results}
     choice = min(results, key=lambda r: r["compress_ms"] + r["decompress_ms"])["knobs"]
     entry["choice"] = dict(choice)
@@ -259,7 +290,8 @@ def _tune_batch(torch, lib, fields, label, reps, rel=1e-3):
     out = torch.empty(cap, dtype=torch.uint8, device=fields[0].device)
     dec = torch.empty(sum(f.numel() for f in fields), dtype=fields[0].dtype, device=fields[0].device)
     results = []
-    for cand in BATCH_CANDIDATES:
+    cls = batch_class(shapes, itemsize)
+    for cand in candidates(BATCH_CANDIDATES, cls["dtype"]):
         lib.waltz_b200_batch_config(cand["mode"], cand["width"])
         set_single(lib, batch_single_knobs(cand))
         arcs = waltz_b200.compress_batch(fields, bounds, out=out, tuned=False)
@@ -270,7 +302,7 @@ def _tune_batch(torch, lib, fields, label, reps, rel=1e-3):
     lib.waltz_b200_batch_config(*[DEFAULT_BATCH[k] for k in ("mode", "width")])
     set_single(lib, {})
     choice = min(results, key=lambda r: r["compress_ms"] + r["decompress_ms"])["knobs"]
-    return {"class": batch_class(shapes, itemsize), "workload": label, "measured": results, "choice": dict(choice)}
+    return {"class": cls, "workload": label, "measured": results, "choice": dict(choice)}
 
 
 def tune(quick=False, reps=5, path=TABLE):
