@@ -87,6 +87,8 @@ def test_candidates_differ_in_acting_knobs_only():
     assert {c["small_inv"] for c in f64} == {1 << 15, 1 << 18, 1 << 21, 1 << 24, 1 << 27}
     plane = A.candidates(A.SINGLE_CANDIDATES, "f32", "plane")
     assert all("zmarch" not in c and "small_march" not in c for c in plane) and len(plane) == 2 * 3 * 4
+    marches = A.candidates([{**c, "xy_march": 3} for c in A.SINGLE_CANDIDATES], "f32", "plane")
+    assert marches == [{"stage_kernels": 1, "xy_march": 3}, {"stage_kernels": 0, "xy_march": 3}]
     batch = A.candidates(A.BATCH_CANDIDATES, "f32")
     assert all("small_march" not in c for c in batch) and len(batch) < len(A.BATCH_CANDIDATES)
     assert any(c.get("small_march") for c in A.candidates(A.BATCH_CANDIDATES, "f64"))

@@ -104,7 +104,8 @@ def acting(knobs, dtype, schedule=None):
        larger of small_fwd and small_march_fwd, their inverse levels, of
        doubles only, up to the larger of small_inv and small_march (float ones
        are staged at every size);
-     * plane fields have no dyadic z-march and no dyadic levels;
+     * plane fields have no dyadic z-march and no dyadic levels, and no
+       threshold acts in the direction that xy_march takes as a whole;
      * a batch of floats has no inverse level that small_march acts on."""
     k = {**DEFAULT_SINGLE, **knobs}
     if schedule == "dyadic":
@@ -113,7 +114,12 @@ def acting(knobs, dtype, schedule=None):
             a["small_inv"] = max(k["small_inv"], k["small_march"])
         return a
     if schedule == "plane":
-        return {n: k[n] for n in ("stage_kernels", "small_inv", "small_fwd", "xy_march")}
+        a = {"stage_kernels": k["stage_kernels"], "xy_march": k["xy_march"]}
+        if not k["xy_march"] & 1:
+            a["small_fwd"] = k["small_fwd"]
+        if not k["xy_march"] & 2:
+            a["small_inv"] = k["small_inv"]
+        return a
     return {n: v for n, v in knobs.items() if n != "small_march" or dtype == "f64"}
 
 
