@@ -54,13 +54,29 @@ def test_extrema_at_any_alignment(n, offset, dtype):
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 def test_matrix_repairs_with_a_partial_last_warp(form, dtype):
     """612 columns: the last warp of the matrix synthesis holds four of them.
-    Every sample meets the bound and the decode repeats."""
+    The repairs recorded are exactly the samples whose synthesis without
+    repairs misses the bound, each with its error; every sample meets the
+    bound and the decode repeats."""
     import waltz_b200
     from waltz_b200 import synthetic as S
     a = S.power_law_field((33, 18, 34), 6, dtype=dtype)
     eb = float(np.float32(1e-3))
     archive = waltz_b200.compress(a, abs_error=eb, form=form)
-    assert int.from_bytes(archive[24:28], "little") > 0, "the field has repairs"
+    wzp, = np.frombuffer(archive[16:24], np.uint64)
+    count, outliers = np.frombuffer(archive[24:32], np.uint32)
+    assert count > 0, "the field has repairs"
+    at = 32 + (int(wzp) + 7) // 8 * 8
+    values = at + (4 * int(count) + 7) // 8 * 8
+    rest = values + (a.itemsize * int(count) + 7) // 8 * 8
+    # the same archive without its repair section
+    bare = archive[:4] + bytes(4) + archive[8:24] + bytes(4) + archive[28:at] + archive[rest:]
+    raw = waltz_b200.decompress(bare, shape=a.shape, dtype=dtype)
+    err = (raw - a).ravel()
+    missed = np.flatnonzero(np.abs(err) > dtype(eb))
+    index = np.frombuffer(archive[at:at + 4 * count], np.uint32)
+    assert np.array_equal(index, missed)
+    assert np.array_equal(np.frombuffer(archive[values:values + a.itemsize * count], dtype), err[missed])
+    assert (index % 612 >= 608).any(), "some of them in the last warp"
     out = waltz_b200.decompress(archive, shape=a.shape, dtype=dtype)
     assert np.abs(out.astype(np.float64) - a.astype(np.float64)).max() <= eb
     assert waltz_b200.decompress(archive, shape=a.shape, dtype=dtype).tobytes() == out.tobytes()

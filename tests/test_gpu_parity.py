@@ -662,9 +662,11 @@ def test_unaligned_archive_addresses():
 def test_dyadic_small_levels_as_marches_match_oracle(nxyz, dtype, small_march):
     """Dyadic fields whose small levels (every level, with the largest
     threshold, the finest one's repair and final emitters included) run as
-    marches: the inverse as a Z march then an XY march instead of the tile
-    inverse, the forward as an XY march then a Z march instead of the
-    z-march. Transforms, archives and decodes equal the oracle's."""
+    marches: the forward as an XY march then a Z march instead of the z-march
+    and, for doubles, the inverse as a Z march then an XY march instead of the
+    tile inverse. (Float inverse levels march where the copy engine cannot
+    stage them, as in the second and fourth field.) Transforms, archives and
+    decodes equal the oracle's."""
     import torch
     import waltz_b200
     from waltz_b200 import autotune as A
