@@ -204,7 +204,7 @@ static thread_local Options t_opt;
 // Polls of the float inverse levels' copy waits (a test hook lowers it).
 static thread_local uint32_t t_copy_polls = kWaitBound;
 
-// One Z level of the plane schedule as a per-column register march
+// One Z level, or the Z part of a dyadic one, as a per-column register march
 // (ZMarchOp): a warp per 32 columns and run of windows. A single field's
 // runs are halved until the level has about 32 warps per SM (a run's first
 // window reloads the 4 pairs it shares with the run before); many fields fill
@@ -224,9 +224,10 @@ static void level_z(const Src& src, Dims a, const Out& out, Sink& sink) {
     sink.run<Op>(typename Op::Params{src, a, out, seg, tx}, uint32_t(blocks));
 }
 
-// One XY level of the plane schedule as a warp march (XYMarchOp, taken with
-// WALTZ_B200_OPT_XY_MARCH): a warp per strip of 24 x, plane and run of Y
-// windows; runs halved for a single field until the level has about 32
+// One XY level, or the X and Y part of a dyadic one, as a warp march
+// (XYMarchOp): plane levels with WALTZ_B200_OPT_XY_MARCH, small levels and
+// levels the copy engine cannot stage. A warp per strip of 56 x, plane and run
+// of Y windows; runs halved for a single field until the level has about 32
 // warps per SM, as for the Z levels.
 template <class T, bool Inverse, class Src, class Out>
 static void level_xy(const Src& src, Dims a, const Out& out, Sink& sink) {
@@ -332,8 +333,8 @@ static bool level_fwd_stream(const FwdSrc<T>& src, Dims a, const FwdOut<T>& out,
 template <class T>
 static void level_fwd_march(const FwdSrc<T>& src, Dims a, const FwdOut<T>& out, T* tmp, Sink& sink) {
     const size_t ty = a.x, tz = size_t(a.x) * a.y;
-    level_xy<T, false>(src, a, FwdOut<T>{tmp, ty, tz, nullptr, halve(a, AX | AY), a, AX | AY}, sink);
-    level_z<T, false>(FwdSrc<T>{tmp, ty, tz}, a, FwdOut<T>{out.dst, out.sy, out.sz, out.low, out.lo, a, AZ}, sink);
+    level_xy<T, false>(src, a, FwdOut<T>{tmp, ty, tz, nullptr, halve(a, AX | AY)}, sink);
+    level_z<T, false>(FwdSrc<T>{tmp, ty, tz}, a, FwdOut<T>{out.dst, out.sy, out.sz, out.low, out.lo}, sink);
 }
 
 // One dyadic inverse level from TMA-staged parity boxes (float: the y-march
@@ -588,7 +589,7 @@ static void forward(const Geometry& g, const T* in, T* C, T* lowA, T* lowB, T* i
             // marches through `inter` (unused by the dyadic schedule): at
             // 301 x 333 x 325 f32 the finest level takes 0.145 ms so and
             // took 0.279 with tiles staged by reflecting loads
-            const FwdOut<T> out{C, sy, sz, last ? nullptr : lows[l & 1], lo, a, AX | AY | AZ};
+            const FwdOut<T> out{C, sy, sz, last ? nullptr : lows[l & 1], lo};
             if (vol(a) <= std::max(t_opt.small_march_fwd, t_opt.small_fwd) ||
                 !level_fwd_stream<T>(src, a, out, status, sink))
                 level_fwd_march<T>(src, a, out, inter, sink);
@@ -609,7 +610,7 @@ static void forward(const Geometry& g, const T* in, T* C, T* lowA, T* lowB, T* i
     for (unsigned l = 0; l < (matrix || zstage ? 0u : g.lz); ++l) {
         const Dims a = g.zl[l], lo = halve(a, AZ);
         const bool last = l + 1 == g.lz;
-        FwdOut<T> out{zdst, sy, sz, last ? nullptr : lows[l & 1], lo, a, AZ};
+        FwdOut<T> out{zdst, sy, sz, last ? nullptr : lows[l & 1], lo};
         level_z<T, false>(src, a, out, sink);
         src = FwdSrc<T>{lows[l & 1], lo.x, size_t(lo.x) * lo.y};
     }
@@ -623,7 +624,7 @@ static void forward(const Geometry& g, const T* in, T* C, T* lowA, T* lowB, T* i
     for (unsigned l = 0; l < g.lxy; ++l) {
         const Dims a = g.xyl[l], lo = halve(a, AX | AY);
         const bool last = l + 1 == g.lxy;
-        FwdOut<T> out{C, sy, sz, last ? nullptr : lows[l & 1], lo, a, AX | AY};
+        FwdOut<T> out{C, sy, sz, last ? nullptr : lows[l & 1], lo};
         if ((t_opt.xy_march & 1u) || vol(a) <= t_opt.small_fwd ||
             !level_fwd_stream<T, false>(src, a, out, status, sink))
             level_xy<T, false>(src, a, out, sink);
@@ -1610,8 +1611,8 @@ struct PinnedBuffer {
     }
 };
 
-// CTAs of an extrema launch: four per SM (all resident, 32 warps each SM at
-// 512 threads) as far as every thread has its four vectors.
+// CTAs of an extrema launch: four per SM (all resident: 64 warps an SM at 512
+// threads) as far as every thread has its four vectors.
 constexpr unsigned kExtremaBlocks = 148 * 4;
 
 template <class T>

@@ -122,7 +122,6 @@ __host__ __device__ inline uint32_t mirror(int64_t p, uint32_t n) {
 __host__ __device__ inline uint32_t split_of(uint32_t r, uint32_t n) {
     return (r >> 1) + ((r & 1) ? half_len(n) : 0);
 }
-__host__ __device__ inline uint32_t coeff_at(int64_t p, uint32_t n) { return split_of(mirror(p, n), n); }
 
 inline unsigned levels_of(uint32_t length) {
     unsigned l = 0;

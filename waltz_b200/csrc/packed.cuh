@@ -31,6 +31,8 @@ __device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
 // product as a multiply-add of -0 is contracted too). A product that feeds only
 // a sum therefore has to be formed with the scalar __fmul_rn; in the lifting
 // every scaled sample is also the addend of a multiply-add and stays a product.
+// Another assembler may contract otherwise: the parity tests against the oracle
+// hold every form that uses this file to the exact bits.
 __device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
     f2 r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));

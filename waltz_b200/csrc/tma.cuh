@@ -101,8 +101,8 @@ inline EncodeTiledFn encode_tiled() {
 
 // 3-D tiled map of a T array with x fastest (strides in elements). Returns
 // false when the array does not meet the copy engine's rules (16-byte base
-// and row strides) or the encoder is unavailable; callers then stage with
-// ordinary loads.
+// and row strides) or the encoder is unavailable; the level then runs as
+// register marches.
 template <class T>
 inline bool make_map_3d(CUtensorMap* map, const T* base, uint64_t nx, uint64_t ny, uint64_t nz, uint64_t sy,
                         uint64_t sz, uint32_t bx, uint32_t by, uint32_t bz,

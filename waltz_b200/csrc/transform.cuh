@@ -49,22 +49,6 @@ template <class T> struct FwdOut {
     size_t sy, sz;
     T* low;
     Dims lo;
-    Dims a;
-    int mask;
-    __device__ __forceinline__ void operator()(uint32_t x, uint32_t y, uint32_t z, T v) const {
-        const bool ex = !(mask & AX) || !(x & 1), ey = !(mask & AY) || !(y & 1), ez = !(mask & AZ) || !(z & 1);
-        const uint32_t cx = (mask & AX) ? split_of(x, a.x) : x;
-        const uint32_t cy = (mask & AY) ? split_of(y, a.y) : y;
-        const uint32_t cz = (mask & AZ) ? split_of(z, a.z) : z;
-        if (low && ex && ey && ez) low[(size_t(cz) * lo.y + cy) * lo.x + cx] = v;
-        else dst[size_t(cz) * sz + size_t(cy) * sy + cx] = v;
-    }
-    // All-axes form with the column's split (cx, cy) resolved by the caller.
-    __device__ __forceinline__ void put(uint32_t cx, uint32_t cy, bool even_xy, uint32_t z, T v) const {
-        const uint32_t cz = split_of(z, a.z);
-        if (low && even_xy && !(z & 1)) low[(size_t(cz) * lo.y + cy) * lo.x + cx] = v;
-        else dst[size_t(cz) * sz + size_t(cy) * sy + cx] = v;
-    }
 };
 
 // Inverse output into a compact or strided array.

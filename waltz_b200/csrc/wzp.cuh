@@ -483,7 +483,7 @@ template <class T> struct QuantBricks {
     }
 };
 
-// Bound by the ALU pipe (about 60 instructions per sample, seven barriers a
+// Bound by the ALU pipe (about 60 instructions per sample, six barriers a
 // chunk; four CTAs per SM overlap them). 512^3 f32: 0.41 ms (2.9 TB/s of read,
 // rewrite and archive); 0.50 ms with per-sample masks, shift-network compress
 // and fourteen barriers a chunk.
@@ -940,7 +940,7 @@ template <class T> struct WzpDecodeArgs {
     uint32_t* status;
 };
 
-// Bound like the encoder (52 instructions per sample, six barriers). 512^3
+// Bound like the encoder (52 instructions per sample, seven barriers). 512^3
 // f32: 0.34 ms; 0.46 ms with a block scan and byte loops per repetition level,
 // shift-network expand and per-sample conversions.
 template <class T> struct WzpDecodeOp {

@@ -1,17 +1,18 @@
-// One Z level of the plane schedule as a per-column march in registers.
+// One Z level of the plane schedule, or the Z part of a dyadic level, as a
+// per-column march in registers.
 //
 // A thread owns one (x, y) column of the level and a run of its Z windows; a
 // warp's 32 lanes take 32 consecutive x of one row, so every load and store
 // of a z row is one 128-byte line and nothing is staged in shared memory.
 // Window w covers outputs [W*w, W*w + W) and reads the P = W/2 + 4 pairs at
 // spatial positions W*w - 4 + 2j (even) and + 1 (odd), reflected at the
-// column's ends exactly as the tile kernels reflect them. Consecutive windows
+// column's ends exactly as the staged kernels reflect them. Consecutive windows
 // share their last / first 4 pairs: those are kept raw in registers, so a
 // later window loads only its W/2 new pairs.
 //  * forward: windows of 16 (the analysis is window independent);
 //  * inverse: the canonical folded windows (16 outputs for float, 8 for
 //    double, origins at multiples of W; cpu/src/transform.cpp:110-147), so
-//    every output takes the arithmetic of the tile kernels' Z pass.
+//    every output takes the arithmetic of the staged kernels' Z pass.
 // Forward sources are checked for finiteness when they carry a status word
 // (the finest level reads every input sample at least once).
 #pragma once
