@@ -477,6 +477,24 @@ def test_work_queue_items_reuse_the_staged_buffers(dtype, shape):
         lib.waltz_b200_batch_config(1, 32)
 
 
+@pytest.mark.parametrize("count", [1, 3, 40])
+def test_batches_split_their_inverse_levels_by_field_count(count):
+    """The float inverse march cuts a field's columns into more CTAs the fewer
+    fields a batch has; archives and decodes stay the single calls'."""
+    torch = _torch()
+    import waltz_b200
+    from waltz_b200 import synthetic as S
+    shape = (64, 88, 96)
+    field = torch.from_numpy(S.power_law_field(shape, 31)).cuda()
+    fields = [field * (1 + k) for k in range(count)]
+    bounds = [float(np.float32(1e-3 * float(f.max() - f.min()))) for f in fields]
+    archives = waltz_b200.compress_batch(fields, bounds)
+    assert bytes(archives[0].cpu().numpy()) == O.compress(fields[0].cpu().numpy(), bounds[0])
+    assert all(torch.equal(a, waltz_b200.compress_tensor(f, eb)) for a, f, eb in zip(archives, fields, bounds))
+    out = waltz_b200.decompress_batch(archives, [shape] * count, torch.float32)
+    assert all(torch.equal(o, waltz_b200.decompress_tensor(a, shape, torch.float32)) for o, a in zip(out, archives))
+
+
 def test_batch_results_are_written_in_place_like_slices():
     """The tensors of a batch decode take in-place operations that autograd
     records, with and without a caller's buffer (here one that does not start

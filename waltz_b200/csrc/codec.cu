@@ -356,16 +356,16 @@ static bool level_inv(const InvSrc<float>& src, Dims a, const Out& out, uint32_t
     p.strips = (a.x + S::SHIFT + S::UX - 1) / S::UX;
     p.zwins = (a.z + S::UZ - 1) / S::UZ;
     const uint64_t columns = uint64_t(p.strips) * p.zwins;
-    // Y windows per CTA: whole columns when many fields fill the GPU; for one
-    // field the split with the fewest steps along its waves of resident CTAs,
-    // a CTA's priming step counted as two thirds of a window (512^3 repair
-    // level: 0.453 ms at 16 windows a CTA, 0.493 at 3, 0.590 at all 64)
+    // Y windows per CTA: the split with the fewest steps along the field's waves
+    // in its share of the resident CTAs, a CTA's priming step counted as two
+    // thirds of a window (512^3 repair level: 0.453 ms at 16 windows a CTA, 0.493
+    // at 3, 0.590 at all 64). A batch of many fields takes whole columns.
     p.seg = wins;
-    if (!sink.many) {
+    {
         static thread_local int device = -1;
         static thread_local size_t granted = 0;
         opt_in_smem(op_kernel_for<Op>(), S::smem, device, granted);
-        const uint64_t slots = resident_slots(op_kernel_for<Op>(), S::smem);
+        const uint64_t slots = std::max<uint64_t>(1, resident_slots(op_kernel_for<Op>(), S::smem) / sink.fields);
         double best = 0;
         for (uint32_t k = 1; k <= 32 && k <= wins; ++k) {
             const uint32_t seg = (wins + k - 1) / k;
@@ -1780,7 +1780,7 @@ static void capture_stage_batched(BatchStreams& bs, int groups, CachedGraph& cg,
     for (uint32_t i = 0; i < count; ++i) {
         Recorder& rec = recs[i % uint32_t(groups)];
         rec.begin_field();
-        Sink sink{bs.cap, &rec, true};
+        Sink sink{bs.cap, &rec, true, count};
         enqueue(i, sink);
     }
     std::vector<BatchPlan> plans;

@@ -186,6 +186,7 @@ struct Sink {
     cudaStream_t stream = nullptr;
     Recorder* rec = nullptr;
     bool many = false; // many fields share the GPU: prefer fewer, larger blocks of work per field
+    uint32_t fields = 1; // how many of them
     bool chained = false; // one field's stages, not captured: each launched ahead of its predecessor's end
     template <class Op> void run(const typename Op::Params& p, uint32_t blocks, size_t smem = 0) {
         if (rec) rec->add(std::make_unique<OpRec<Op>>(p, blocks, smem));
