@@ -359,7 +359,7 @@ static bool level_inv(const InvSrc<float>& src, Dims a, const Out& out, uint32_t
     // Y windows per CTA: the split with the fewest steps along the field's waves
     // in its share of the resident CTAs, a CTA's priming step counted as two
     // thirds of a window (512^3 repair level: 0.453 ms at 16 windows a CTA, 0.493
-    // at 3, 0.590 at all 64). A batch of many fields takes whole columns.
+    // at 3, 0.590 at all 64). Fields with one slot or less take whole columns.
     p.seg = wins;
     {
         static thread_local int device = -1;
@@ -367,7 +367,7 @@ static bool level_inv(const InvSrc<float>& src, Dims a, const Out& out, uint32_t
         opt_in_smem(op_kernel_for<Op>(), S::smem, device, granted);
         const uint64_t slots = std::max<uint64_t>(1, resident_slots(op_kernel_for<Op>(), S::smem) / sink.fields);
         double best = 0;
-        for (uint32_t k = 1; k <= 32 && k <= wins; ++k) {
+        for (uint32_t k = 1; slots > 1 && k <= 32 && k <= wins; ++k) {
             const uint32_t seg = (wins + k - 1) / k;
             const uint64_t blocks = columns * ((wins + seg - 1) / seg);
             const double steps = double((blocks + slots - 1) / slots) * (seg + 0.67);
